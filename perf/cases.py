@@ -203,3 +203,67 @@ def tolerance(case):
     if case["kind"] == "bias":
         return {"rel": 7e-3, "max": 0.04}
     return {"rel": 1.2e-2, "max": 0.1}
+
+
+def _attention64(q, k, v, valid, bias, grad):
+    """Attention of q [B, Hq, Sq, 128] over k, v [B, Hkv, Skv, 128] in 64 bits, a block of query rows at a time: o and
+    lse [B * Hq, Sq], and with an upstream gradient dq, dk, dv."""
+    B, Hq, Sq, _ = q.shape
+    per_kv = Hq // k.shape[1]
+    o, lse = torch.empty_like(q), q.new_empty(B, Hq, Sq)
+    grads = [torch.zeros_like(t) for t in (q, k, v)] if grad is not None else []
+    step = max(1, (1 << 27) // k.shape[2])
+    for b in range(B):
+        n = valid[b] if valid is not None else k.shape[2]
+        for h in range(Hq):
+            kh, vh = k[b, h // per_kv, :n], v[b, h // per_kv, :n]
+            for i in range(0, Sq, step):
+                rows = slice(i, min(i + step, Sq))
+                scores = q[b, h, rows] @ kh.T * SCALE
+                if bias is not None:
+                    scores += bias[0, 0, rows, :n]
+                lse[b, h, rows] = torch.logsumexp(scores, -1)
+                p = scores.sub_(lse[b, h, rows, None]).exp_()
+                o[b, h, rows] = p @ vh
+                if grad is not None:
+                    dq, dk, dv = grads
+                    do = grad[b, h, rows]
+                    dv[b, h // per_kv, :n] += p.T @ do
+                    ds = p.mul_(do @ vh.T - (do * o[b, h, rows]).sum(-1, keepdim=True)).mul_(SCALE)
+                    dq[b, h, rows] = ds @ kh
+                    dk[b, h // per_kv, :n] += ds.T @ q[b, h, rows]
+    return [o, lse.view(B * Hq, Sq), *grads]
+
+
+def _layer64(case, s):
+    Hq, Hkv = case["Hq"], case["Hkv"]
+    module, eps = s["module"], s["module"].q_norm.variance_epsilon
+    leaves = {"x": s["x"], **dict(module.named_parameters())}
+    leaves = {name: t.detach().double().requires_grad_() for name, t in leaves.items()}
+
+    def heads(t, weight, n):
+        return (t @ weight.T).view(1, -1, n, 128).transpose(1, 2)
+
+    def norm(t, weight):
+        return weight * t * torch.rsqrt(t.pow(2).mean(-1, keepdim=True) + eps)
+
+    states = s["states"].double()
+    q = norm(heads(leaves["x"], leaves["q_proj.weight"], Hq), leaves["q_norm.weight"])
+    k = norm(heads(states, leaves["k_proj.weight"], Hkv), leaves["k_norm.weight"])
+    v = heads(states, leaves["v_proj.weight"], Hkv)
+    grad = s["grad"].double()
+    d_attn = heads(grad, leaves["o_proj.weight"].detach().T, Hq)
+    o, _, dq, dk, dv = _attention64(q.detach(), k.detach(), v.detach(), None, None, d_attn)
+    attn = o.transpose(1, 2).reshape(1, -1, Hq * 128)
+    out = attn @ leaves["o_proj.weight"].T
+    return [out.detach(), *torch.autograd.grad((q, k, v, out), list(leaves.values()), (dq, dk, dv, grad))]
+
+
+def exact(case, seed):
+    s = prepare(case, seed)
+    if s["kind"] == "layer":
+        return _layer64(case, s)
+    bias = _image_bias(s["image_of_key"], s["images_before"]).double() if s["kind"] == "bias" else None
+    q, k, v = (s[n].detach().double() for n in "qkv")
+    o, lse, *grads = _attention64(q, k, v, s["valid"], bias, s["grad"].double() if case["backward"] else None)
+    return [o, *grads] if case["backward"] else [o, lse]
