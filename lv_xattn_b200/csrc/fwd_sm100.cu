@@ -454,19 +454,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
 }
 
 // ---------------------------------------------------------------------------------------------
-static int g_num_sms = 0;
-static int num_sms() {
-  if (!g_num_sms) {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0)
-      g_num_sms = n;
-    else
-      g_num_sms = 148;
-  }
-  return g_num_sms;
-}
-
 FwdPlan plan_fwd(const lvx_shape& s) {
   FwdPlan p;
   const int g = s.Hq / s.Hkv;
@@ -478,7 +465,10 @@ FwdPlan plan_fwd(const lvx_shape& s) {
   const int sms = 148;  // plan for the full part; a fixed figure keeps the workspace size device-independent
   int best = 1;
   double best_cost = 1e300;
-  const int max_split = p.kv_tiles < 64 ? (p.kv_tiles > 0 ? p.kv_tiles : 1) : 64;
+  // With few rows the partials are small and a single KV slab may need every SM: one split per SM at most. Above that,
+  // 64 splits keep the combine kernel's walk and the partials (nsplit * 520 bytes per row) in bounds.
+  const int cap = p.rows <= kFewRows && qb == 1 ? sms : 64;
+  const int max_split = p.kv_tiles < cap ? (p.kv_tiles > 0 ? p.kv_tiles : 1) : cap;
   for (int ns = 1; ns <= max_split; ++ns) {
     const long ctas = base * ns;
     const long waves = (ctas + sms - 1) / sms;
@@ -504,7 +494,8 @@ int launch_fwd_block(const lvx_shape& s, const FwdPlan& pl, const void* q, const
                      cudaStream_t st, const lvx_block_wait* bw) {
   if (!(sm_scale > 0.f)) return fail(LVX_ERR_SHAPE, "lvx_fwd_block: sm_scale must be positive");
   if (s.dtype == LVX_FP32) return launch_fwd_block_fp32(s, pl, q, k, v, kv_valid_len, sm_scale, o_part, ml_part, st);
-  (void)num_sms;
+  if (pl.rows <= kFewRows && q_blocks_of(s) == 1 && bw == nullptr)
+    return launch_fwd_rows(s, pl, q, k, v, kv_valid_len, sm_scale, o_part, ml_part, status, st);
   CUtensorMap tmQ, tmK, tmV;
   const int es = elt_size(s.dtype);
   const uint64_t row_bytes = uint64_t(128) * es;

@@ -44,6 +44,12 @@ FwdPlan plan_fwd(const lvx_shape& s);
 int launch_fwd_block(const lvx_shape& s, const FwdPlan& p, const void* q, const void* k, const void* v,
                      const int32_t* kv_valid_len, float sm_scale, float* o_part, float* ml_part, int* status,
                      cudaStream_t st, const lvx_block_wait* bw = nullptr);
+// The forward block for few packed query rows (fwd_rows_sm100.cu); same plan and partials layout. Measured at one token
+// over 409,856 keys: 270 us a call against 447 with the 256-row kernel.
+constexpr int kFewRows = 64;
+int launch_fwd_rows(const lvx_shape& s, const FwdPlan& p, const void* q, const void* k, const void* v,
+                    const int32_t* kv_valid_len, float sm_scale, float* o_part, float* ml_part, int* status,
+                    cudaStream_t st);
 int launch_fwd_combine(const lvx_shape& s, const FwdPlan& p, const float* o_part, const float* ml_part,
                        const float* o_in, const float* lse_in, void* o_out, float* lse_out, int out_is_final,
                        cudaStream_t st);

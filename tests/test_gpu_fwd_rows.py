@@ -1,0 +1,43 @@
+"""The forward kernel for few packed query rows (g * Sq <= 64) at the edges of its tiles: 16-row groups, 128-key tiles,
+key ranges that are empty or end inside a tile, scores that force a rescale. Bars as in test_gpu_fwd.py."""
+import math
+
+import pytest
+import torch
+
+import _parity
+from oracle import attention_oracle as orc
+
+pytestmark = pytest.mark.gpu
+SCALE = 1.0 / math.sqrt(128.0)
+
+
+def run_and_check(device, B, Hq, Hkv, Sq, Skv, dtype, valid=None, gain=1.0, label=""):
+    from lv_xattn_b200 import ops, _lib
+    q, k, v, _ = orc.make_inputs(B, Hq, Hkv, Sq, Skv, 128, 11, dtype)
+    q = q * gain
+    o_ref, lse_ref = orc.attention_fwd(q, k, v, SCALE, valid)
+    kvl = None if valid is None else torch.tensor(valid, dtype=torch.int32, device=device)
+    o, lse = ops.fwd_block(q.to(device), k.to(device), v.to(device), SCALE, kv_valid_len=kvl)
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    _parity.assert_lse_close(lse.cpu().view(B, Hq, Sq), lse_ref, label)
+    _parity.assert_close(o.float().cpu(), o_ref, "o", label, *_parity.BF16["o"])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("heads,Sq", [((1, 1), 1), ((4, 1), 4), ((1, 1), 17), ((4, 2), 16), ((3, 1), 11), ((4, 1), 16),
+                                      ((5, 1), 13)])      # 1, 16, 17, 32, 33, 64 and 65 (the other kernel) rows
+def test_row_groups(cuda_device, heads, Sq, dtype):
+    run_and_check(cuda_device, 2, heads[0], heads[1], Sq, 1601, dtype, label=f"rows{heads}{Sq}{dtype}")
+
+
+@pytest.mark.parametrize("skv", [1, 15, 127, 128, 129, 5 * 128 + 77, 40961])
+def test_key_edges(cuda_device, skv):
+    run_and_check(cuda_device, 1, 8, 2, 3, skv, torch.bfloat16, label=f"rows_keys{skv}")
+
+
+@pytest.mark.parametrize("Sq", [2, 8, 16])
+def test_key_padding_and_large_scores(cuda_device, Sq):
+    # a sample without any valid key, ranges that end inside a warp's keys; queries scaled so that the running max jumps
+    run_and_check(cuda_device, 4, 4, 1, Sq, 900, torch.bfloat16, valid=[900, 0, 387, 5], gain=16.0, label=f"rows_pad{Sq}")
