@@ -132,9 +132,9 @@ typedef struct lvx_bias {
   int64_t stride_block, stride_b, stride_h, stride_q, stride_kv;
 } lvx_bias;
 
-/* lvx_fwd_block / lvx_bwd_block with a dense bias (any dtype). These run the library's general FP32-FMA block
- * kernels instead of the tensor-core ones (key padding expressed as kv_valid_len stays on the tensor-core path);
- * same workspace, outputs and accumulate modes. */
+/* lvx_fwd_block / lvx_bwd_block with a dense bias (any dtype). 16-bit forwards and bf16 backwards run the tensor-core
+ * kernels with P and dS in two 16-bit parts, fp32 and the fp16 backward the general kernels; same workspace, outputs and
+ * accumulate modes. */
 int lvx_fwd_block_bias(const lvx_shape* s, const void* q, const void* k, const void* v,
                        const int32_t* kv_valid_len, const lvx_bias* bias, float sm_scale, void* workspace,
                        size_t workspace_bytes, void* stream);

@@ -18,7 +18,7 @@ at home and travels instead of O (:926-942 recomputes it on every rank), K/V are
 count (no expansion, :392-393), and key padding has a native form (a per-batch valid length, handled inside the
 tensor-core kernels). The reference's general bias protocol -- bias_func(*local_bias_args, *remote_bias_args),
 the remote arguments travelling with the query block (:359-360, :373-374, :386-389) -- is kept: with a bias_func
-the step loop runs one block per step and the block kernels are the general FP32-FMA ones.
+the step loop runs one block per step and the block kernels are those that take a bias.
 """
 from __future__ import annotations
 
@@ -119,7 +119,7 @@ def _build_bias(bias_func, local_bias_args, peer_bias_args, q, k):
     """The reference's bias protocol (lv_xattn/attn.py:386-389): the additive bias of one step is
     bias_func(*local_bias_args, *peer_bias_args) -> [B, 1 or H, Sq_local, Skv_local], where the local arguments
     belong to this rank's K/V shard and the peer arguments arrived with the query block. It is added to the scaled
-    scores (S = sm_scale*q.k + bias); steps with a bias run the general FP32-FMA kernels."""
+    scores (S = sm_scale*q.k + bias)."""
     if bias_func is None:
         return None
     bias = bias_func(*(list(local_bias_args) + list(peer_bias_args)))

@@ -286,8 +286,10 @@ int lvx_fwd_block_bias(const lvx_shape* s, const void* q, const void* k, const v
                 p.o_part_bytes + p.ml_part_bytes);
   float* o_part = static_cast<float*>(workspace);
   float* ml_part = reinterpret_cast<float*>(static_cast<char*>(workspace) + p.o_part_bytes);
-  return launch_fwd_block_simt(*s, p, q, k, v, kv_valid_len, bias, sm_scale, o_part, ml_part,
-                               static_cast<cudaStream_t>(stream));
+  int* sp = status_ptr();
+  if (!sp) return fail(LVX_ERR_DRIVER, "%s: status word unavailable", who);
+  return launch_fwd_block(*s, p, q, k, v, kv_valid_len, sm_scale, o_part, ml_part, sp, static_cast<cudaStream_t>(stream),
+                          nullptr, bias);
 }
 
 int lvx_bwd_block_bias(const lvx_shape* s, const void* q, const void* d_o, const float* lse, const float* delta,
@@ -311,8 +313,10 @@ int lvx_bwd_block_bias(const lvx_shape* s, const void* q, const void* d_o, const
   LVX_REQUIRE_PTR(v, who);
   LVX_REQUIRE_PTR(dk_acc, who);
   LVX_REQUIRE_PTR(dv_acc, who);
-  return launch_bwd_block_simt(*s, q, d_o, lse, delta, k, v, kv_valid_len, bias, sm_scale, dq_acc, dk_acc, dv_acc,
-                               accumulate_dkdv, static_cast<cudaStream_t>(stream));
+  int* sp = status_ptr();
+  if (!sp) return fail(LVX_ERR_DRIVER, "%s: status word unavailable", who);
+  return launch_bwd_block(*s, q, d_o, lse, delta, k, v, kv_valid_len, sm_scale, dq_acc, static_cast<float*>(dk_acc),
+                          static_cast<float*>(dv_acc), accumulate_dkdv, sp, static_cast<cudaStream_t>(stream), nullptr, bias);
 }
 
 int lvx_kv_project(int dtype, const void* x, const void* wk, const void* wv, const void* norm_w, float eps, int batch,

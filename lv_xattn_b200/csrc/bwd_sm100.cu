@@ -40,10 +40,17 @@
 //               per 60-75 cycles, so eight warps are needed)
 //   warp  24    TMA producer: K,V once; Q,dO tiles through a 2-stage ring
 //   warp  25    tcgen05.mma issuer; owns the TMEM allocation
+//
+// The BIAS form (dense additive fp32 bias on the scores, bf16 inputs) keeps P and dS as the sum of two bf16 numbers:
+// both were fp32 before this path used the tensor core. P^T then fills X completely (high halves in its first 64
+// columns, low halves in the rest) and dS^T takes two shared-memory tiles, which leaves one buffer for dO instead of
+// two (dO of tile j is free after dV(j), so its successor still arrives under the dS^T half). dV, dK and dQ^T take
+// 16 MMAs instead of 8. The transposed frame suits the bias: a warp's lanes are 32 consecutive keys, so a column's bias
+// values are one 128-byte read. fp16 stays with the FP32-FMA kernel: dS has no bound there, and half of it could
+// fall among fp16's subnormals. Measured at 32 heads, 512 x 6,404: 436 us, 5,177 on the FP32-FMA kernel.
 #include "lvx_internal.h"
 #include "sm100_prims.cuh"
 #include "block_wait.cuh"
-#include <cuda_fp16.h>
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -58,6 +65,9 @@ constexpr int BWD_OFF_K = 0;
 constexpr int BWD_OFF_V = BWD_TILE;
 constexpr int BWD_OFF_Q = 2 * BWD_TILE;                          // stage s: Q at +s*2*TILE, dO right after
 constexpr int BWD_OFF_DS = BWD_OFF_Q + BWD_NSQ * 2 * BWD_TILE;
+// BIAS: Q stage s at BWD_OFF_Q + s*TILE, then dO, then dS^T (high halves, low halves)
+constexpr int BWD_OFF_DO_B = BWD_OFF_Q + 2 * BWD_TILE;
+constexpr int BWD_OFF_DS_B = BWD_OFF_Q + 3 * BWD_TILE;
 constexpr int BWD_OFF_STAT = BWD_OFF_DS + BWD_TILE;              // [2][lse2 128 | delta 128]
 constexpr int BWD_OFF_BAR = BWD_OFF_STAT + 2 * 256 * 4;
 constexpr int BWD_SMEM = BWD_OFF_BAR + 256;
@@ -85,7 +95,9 @@ enum {
   BB_ACC_DONE,
   BB_DRAIN,
   BB_STAT_FULL,                        // x2
-  BB_COUNT = BB_STAT_FULL + 2
+  BB_DO_FULL = BB_STAT_FULL + 2,       // BIAS only: dO has a single buffer and barriers of its own
+  BB_DO_EMPTY,
+  BB_COUNT
 };
 
 struct BwdParams {
@@ -106,6 +118,7 @@ struct BwdParams {
   float* dv_acc;
   int accumulate;      // 0 overwrite fp32, 1 add to fp32, 2 write the finished gradient in the input dtype
   BlockWait bw;        // query blocks that may still be arriving from other ranks
+  BiasView bias;       // BIAS kernel only
   int* status;
 };
 
@@ -124,13 +137,7 @@ __device__ long long g_bwd_ts[2 * 8 * 16];
 
 #define BWD_CODE(role, bar) (LVX_DEV_TIMEOUT_BASE | 0x200 | ((role) << 5) | (bar))
 
-template <bool IS_BF16>
-__device__ __forceinline__ float2 unpack16x2(uint32_t v) {
-  if (IS_BF16) return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
-  return __half22float2(*reinterpret_cast<const __half2*>(&v));
-}
-
-template <bool IS_BF16>
+template <bool IS_BF16, bool BIAS>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
            const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const BwdParams p) {
@@ -179,6 +186,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     mbar_init(&bars[BB_ACC_DONE], 1);
     mbar_init(&bars[BB_DRAIN], 1);
     for (int b = 0; b < 2; ++b) mbar_init(&bars[BB_STAT_FULL + b], 8);   // warps 0-7 publish
+    mbar_init(&bars[BB_DO_FULL], 1);
+    mbar_init(&bars[BB_DO_EMPTY], 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -259,6 +268,33 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           float stat_after = 0.f;
           if (j + 2 < ntot) stat_after = fetch_stat(j + 2);
           if (warp == 0) BWD_TS(0, 0);
+          // The bias of this key (lane) for the warp's 32 query rows: rows run through the heads of the group, so the
+          // address moves by s_q inside a head and by what is left of s_h at its end. Half of the values are requested
+          // before S^T is waited for, the others while the first half is used.
+          const float* bptr = nullptr;
+          int b_left = 0, b_rows = 0;
+          auto bias16 = [&](float (&b)[16]) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              b[i] = 0.f;
+              if (b_rows > 0 && row_valid) b[i] = __ldg(bptr);
+              --b_rows;
+              bptr += p.bias.s_q;
+              if (--b_left == 0) {
+                b_left = p.bias.sq;
+                bptr += p.bias.s_h - p.bias.sq * p.bias.s_q;
+              }
+            }
+          };
+          float bv[BIAS ? 16 : 1];
+          if constexpr (BIAS) {
+            const int row = tile_row0(j) + cg * 32, head = row / p.bias.sq, i0 = row - head * p.bias.sq;
+            bptr = p.bias.base + ((p.bw.first_blk + j / nq) % p.nblk) * p.bias.s_blk + (I.slab / p.hkv) * p.bias.s_b +
+                   ((I.slab % p.hkv) * p.bias.g + head) * p.bias.s_h + i0 * p.bias.s_q + (I.kv0 + r) * p.bias.s_kv;
+            b_left = p.bias.sq - i0;
+            b_rows = p.rows - row;
+            bias16(bv);
+          }
           // ---------------- P^T half: needs S^T only ----------------
           if (!mbar_wait(&bars[BB_S_FULL], jj & 1, abort_flag, p.status, BWD_CODE(0, BB_S_FULL), p.bw.pipe_limit)) {
             alive = false;
@@ -278,10 +314,26 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           }
           const float4* sl = reinterpret_cast<const float4*>(s_stat + (jj & 1) * 256 + cg * 32);
           const float4* sd = reinterpret_cast<const float4*>(s_stat + (jj & 1) * 256 + 128 + cg * 32);
-          uint32_t pk[16];
+          uint32_t pk[16], pl[BIAS ? 16 : 1];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const float4 l2 = sl[i];
+            if constexpr (BIAS) {
+              if (i == 4) bias16(bv);
+              float pe[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float sc = fmaf(bv[(4 * i + e) & 15], 1.4426950408889634f, __uint_as_float(s[4 * i + e]) * c);
+                pe[e] = row_valid ? ex2f(sc - (e == 0 ? l2.x : e == 1 ? l2.y : e == 2 ? l2.z : l2.w)) : 0.f;
+              }
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                pk[2 * i + e] = pack_bf16x2(pe[2 * e], pe[2 * e + 1]);
+                const float2 h = unpack16x2<true>(pk[2 * i + e]);
+                pl[2 * i + e] = pack_bf16x2(pe[2 * e] - h.x, pe[2 * e + 1] - h.y);
+              }
+              continue;
+            }
             float p0 = ex2f(fmaf(__uint_as_float(s[4 * i]), c, -l2.x));
             float p1 = ex2f(fmaf(__uint_as_float(s[4 * i + 1]), c, -l2.y));
             float p2 = ex2f(fmaf(__uint_as_float(s[4 * i + 2]), c, -l2.z));
@@ -297,6 +349,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             break;
           }
           tmem_st16(tX + cg * 16, pk);
+          if constexpr (BIAS) tmem_st16(tX + 64 + cg * 16, pl);
           tc_wait_st();
           tc_fence_before();
           __syncwarp();
@@ -308,7 +361,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           }
           tc_fence_after();
           if (warp == 0) BWD_TS(0, 3);
-          uint32_t dsk[16];
+          uint32_t dsk[16], dsl[BIAS ? 16 : 1];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint32_t dp[16];
@@ -319,13 +372,22 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
               // P is taken back from its packed 16-bit form (the value the dV product uses), which keeps only
               // 16 registers alive across the wait for dP^T
               const float4 dl = sd[h * 4 + i];
-              const float2 pa = unpack16x2<IS_BF16>(pk[h * 8 + 2 * i]), pb = unpack16x2<IS_BF16>(pk[h * 8 + 2 * i + 1]);
+              float2 pa = unpack16x2<IS_BF16>(pk[h * 8 + 2 * i]), pb = unpack16x2<IS_BF16>(pk[h * 8 + 2 * i + 1]);
+              if constexpr (BIAS) {
+                const float2 la = unpack16x2<true>(pl[h * 8 + 2 * i]), lb = unpack16x2<true>(pl[h * 8 + 2 * i + 1]);
+                pa.x += la.x; pa.y += la.y; pb.x += lb.x; pb.y += lb.y;
+              }
               const float d0 = pa.x * (__uint_as_float(dp[4 * i]) - dl.x);
               const float d1 = pa.y * (__uint_as_float(dp[4 * i + 1]) - dl.y);
               const float d2 = pb.x * (__uint_as_float(dp[4 * i + 2]) - dl.z);
               const float d3 = pb.y * (__uint_as_float(dp[4 * i + 3]) - dl.w);
               dsk[h * 8 + 2 * i] = IS_BF16 ? pack_bf16x2(d0, d1) : pack_f16x2(d0, d1);
               dsk[h * 8 + 2 * i + 1] = IS_BF16 ? pack_bf16x2(d2, d3) : pack_f16x2(d2, d3);
+              if constexpr (BIAS) {
+                const float2 ha = unpack16x2<true>(dsk[h * 8 + 2 * i]), hb = unpack16x2<true>(dsk[h * 8 + 2 * i + 1]);
+                dsl[h * 8 + 2 * i] = pack_bf16x2(d0 - ha.x, d1 - ha.y);
+                dsl[h * 8 + 2 * i + 1] = pack_bf16x2(d2 - hb.x, d3 - hb.y);
+              }
             }
           }
           tc_fence_before();
@@ -336,11 +398,15 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             break;
           }
           {
-            uint8_t* rowp = smem + BWD_OFF_DS + (cg >> 1) * BWD_HALF + r * 128;
+            uint8_t* rowp = smem + (BIAS ? BWD_OFF_DS_B : BWD_OFF_DS) + (cg >> 1) * BWD_HALF + r * 128;
 #pragma unroll
             for (int ch = 0; ch < 4; ++ch) {
               uint4 v = make_uint4(dsk[4 * ch], dsk[4 * ch + 1], dsk[4 * ch + 2], dsk[4 * ch + 3]);
               *reinterpret_cast<uint4*>(rowp + ((((cg & 1) * 4 + ch) ^ (r & 7)) << 4)) = v;
+              if constexpr (BIAS) {
+                v = make_uint4(dsl[4 * ch], dsl[4 * ch + 1], dsl[4 * ch + 2], dsl[4 * ch + 3]);
+                *reinterpret_cast<uint4*>(rowp + BWD_TILE + ((((cg & 1) * 4 + ch) ^ (r & 7)) << 4)) = v;
+              }
             }
           }
           fence_async_smem();
@@ -441,7 +507,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         tma_prefetch_desc(&tmDO);
         tma_prefetch_desc(&tmK);
         tma_prefetch_desc(&tmV);
-        int issued = 0, kv_loads = 0;        // Q/dO tiles and K/V tiles requested so far
+        int issued = 0, kv_loads = 0, do_issued = 0;   // Q/dO tiles and K/V tiles requested so far
         bool alive = true;
         int it = 0, jj0 = 0;
         for (int w = blockIdx.x; alive && w < p.nitems; w += gridDim.x) {
@@ -461,13 +527,28 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
               alive = false;
               break;
             }
-            uint8_t* dstq = smem + BWD_OFF_Q + s * 2 * BWD_TILE;
-            mbar_arrive_expect_tx(&bars[BB_Q_FULL + s], 2 * BWD_TILE);
-            for (int h = 0; h < 2; ++h) {
-              tma_load_3d(dstq + h * BWD_HALF, &tmQ, &bars[BB_Q_FULL + s], h * 64, y, qslab);
-              tma_load_3d(dstq + BWD_TILE + h * BWD_HALF, &tmDO, &bars[BB_Q_FULL + s], h * 64, y, qslab);
+            uint8_t* dstq = smem + BWD_OFF_Q + s * (BIAS ? 1 : 2) * BWD_TILE;
+            if constexpr (BIAS) {
+              mbar_arrive_expect_tx(&bars[BB_Q_FULL + s], BWD_TILE);
+              for (int h = 0; h < 2; ++h)
+                tma_load_3d(dstq + h * BWD_HALF, &tmQ, &bars[BB_Q_FULL + s], h * 64, y, qslab);
+              issued = jj + 1;
+              if (!mbar_wait(&bars[BB_DO_EMPTY], (jj & 1) ^ 1, abort_flag, p.status, BWD_CODE(2, BB_DO_EMPTY), p.bw.pipe_limit)) {
+                alive = false;
+                break;
+              }
+              mbar_arrive_expect_tx(&bars[BB_DO_FULL], BWD_TILE);
+              for (int h = 0; h < 2; ++h)
+                tma_load_3d(smem + BWD_OFF_DO_B + h * BWD_HALF, &tmDO, &bars[BB_DO_FULL], h * 64, y, qslab);
+              do_issued = jj + 1;
+            } else {
+              mbar_arrive_expect_tx(&bars[BB_Q_FULL + s], 2 * BWD_TILE);
+              for (int h = 0; h < 2; ++h) {
+                tma_load_3d(dstq + h * BWD_HALF, &tmQ, &bars[BB_Q_FULL + s], h * 64, y, qslab);
+                tma_load_3d(dstq + BWD_TILE + h * BWD_HALF, &tmDO, &bars[BB_Q_FULL + s], h * 64, y, qslab);
+              }
+              issued = jj + 1;
             }
-            issued = jj + 1;
             if (j == 0) {
               // The item's K/V go in after its first Q/dO tile (whose stage frees early): the tile buffers are
               // the previous item's until all of its products have completed.
@@ -493,6 +574,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           };
           if (kv_loads > 0) drain(&bars[BB_KV_FULL], (kv_loads - 1) & 1);
           for (int jj = max(0, issued - BWD_NSQ); jj < issued; ++jj) drain(&bars[BB_Q_FULL + jj % BWD_NSQ], (jj / BWD_NSQ) & 1);
+          if (do_issued > 0) drain(&bars[BB_DO_FULL], (do_issued - 1) & 1);
         }
       }
     } else {
@@ -504,7 +586,11 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         constexpr uint32_t IDESC_DQ = umma_idesc(FMT, UMMA_MN_MAJOR, UMMA_MN_MAJOR, 128, 128);
         constexpr uint32_t HI = umma_desc_hi(1024);
         const uint32_t sK = smem_u32(smem + BWD_OFF_K), sV = smem_u32(smem + BWD_OFF_V);
-        const uint32_t sQ0 = smem_u32(smem + BWD_OFF_Q), sDS = smem_u32(smem + BWD_OFF_DS);
+        const uint32_t sQ0 = smem_u32(smem + BWD_OFF_Q), sDS = smem_u32(smem + (BIAS ? BWD_OFF_DS_B : BWD_OFF_DS));
+        // tile jj's Q and dO; high (and with BIAS low) halves of a product's 16-bit operand pair
+        auto q_at = [&](int jj) { return sQ0 + (jj % BWD_NSQ) * (BIAS ? 1 : 2) * BWD_TILE; };
+        auto do_at = [&](int jj) { return BIAS ? smem_u32(smem + BWD_OFF_DO_B) : q_at(jj) + BWD_TILE; };
+        constexpr int PARTS = BIAS ? 2 : 1;
 
         // D[128 kv, 128 q] = A[128 kv, 128 d] * B[128 q, 128 d]^T, both K-major
         auto issue_st = [&](uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem) {
@@ -519,26 +605,33 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         auto issue_acc = [&](uint32_t d_tmem, uint32_t a_tmem, uint32_t b_smem, bool first) {
           const uint32_t b_lo = umma_desc_lo(b_smem, BWD_HALF);
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            umma_ts_f16(d_tmem, a_tmem + kk * 8, umma_desc_join(b_lo + ((kk * 2048) >> 4), HI), IDESC_ACC,
-                        (!first) || kk > 0);
+          for (int part = 0; part < PARTS; ++part)
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+              umma_ts_f16(d_tmem, a_tmem + part * 64 + kk * 8, umma_desc_join(b_lo + ((kk * 2048) >> 4), HI), IDESC_ACC,
+                          (!first) || kk > 0 || part > 0);
         };
         // dK[128 kv, 128 d] += dS^T[128 kv, 128 q] * Q[128 q, 128 d]: A is the dS^T tile in shared memory read
         // K-major (rows kv, 64-column halves), B is Q read MN-major (rows are q)
         auto issue_dk = [&](uint32_t b_smem, bool first) {
           const uint32_t a_lo = umma_desc_lo(sDS, 16), b_lo = umma_desc_lo(b_smem, BWD_HALF);
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            umma_ss_f16(tmem_base + TM_DK, umma_desc_join(a_lo + (((kk >> 2) * BWD_HALF + (kk & 3) * 32) >> 4), HI),
-                        umma_desc_join(b_lo + ((kk * 2048) >> 4), HI), IDESC_ACC, (!first) || kk > 0);
+          for (int part = 0; part < PARTS; ++part)
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+              umma_ss_f16(tmem_base + TM_DK,
+                          umma_desc_join(a_lo + ((part * BWD_TILE + (kk >> 2) * BWD_HALF + (kk & 3) * 32) >> 4), HI),
+                          umma_desc_join(b_lo + ((kk * 2048) >> 4), HI), IDESC_ACC, (!first) || kk > 0 || part > 0);
         };
         // D[128 d, 128 q] = K^T[128 d, 128 kv] * dS^T[128 kv, 128 q]  (both MN-major: rows are kv)
         const uint32_t kT_lo = umma_desc_lo(sK, BWD_HALF), ds_lo = umma_desc_lo(sDS, BWD_HALF);
         auto issue_dq = [&]() {
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            umma_ss_f16(tmem_base + TM_Y, umma_desc_join(kT_lo + ((kk * 2048) >> 4), HI),
-                        umma_desc_join(ds_lo + ((kk * 2048) >> 4), HI), IDESC_DQ, kk > 0);
+          for (int part = 0; part < PARTS; ++part)
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+              umma_ss_f16(tmem_base + TM_Y, umma_desc_join(kT_lo + ((kk * 2048) >> 4), HI),
+                          umma_desc_join(ds_lo + ((part * BWD_TILE + kk * 2048) >> 4), HI), IDESC_DQ, kk > 0 || part > 0);
         };
 
         bool ok = true;
@@ -555,16 +648,20 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           if (!ok) break;
           tc_fence_after();
           {
-            const uint32_t sQf = sQ0 + (jj0 % BWD_NSQ) * 2 * BWD_TILE;
-            issue_st(tmem_base + TM_X, sK, sQf);
+            issue_st(tmem_base + TM_X, sK, q_at(jj0));
             tc_commit(&bars[BB_S_FULL]);
-            issue_st(tmem_base + TM_Y, sV, sQf + BWD_TILE);
+            if constexpr (BIAS) {
+              ok = mbar_wait(&bars[BB_DO_FULL], jj0 & 1, abort_flag, p.status, BWD_CODE(3, BB_DO_FULL), p.bw.pipe_limit);
+              if (!ok) break;
+              tc_fence_after();
+            }
+            issue_st(tmem_base + TM_Y, sV, do_at(jj0));
             tc_commit(&bars[BB_DP_FULL]);
           }
           for (int j = 0; ok && j < ntot; ++j) {
             const int jj = jj0 + j;
             const int s = jj % BWD_NSQ;
-            const uint32_t sQ = sQ0 + s * 2 * BWD_TILE, sDO = sQ + BWD_TILE;
+            const uint32_t sQ = q_at(jj), sDO = do_at(jj);
             BWD_TS(1, 0);
             // dV needs P^T only, which is published before the dS^T half of the elementwise work; once dV has
             // read X, S^T of the next tile can go there, i.e. while the warps are still producing dS^T
@@ -572,9 +669,10 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             if (!ok) break;
             tc_fence_after();
             issue_acc(tmem_base + TM_DV, tmem_base + TM_X, sDO, j == 0);
+            if constexpr (BIAS) tc_commit(&bars[BB_DO_EMPTY]);     // dP^T and dV of this tile have read dO
             BWD_TS(1, 1);
             const int s1 = (jj + 1) % BWD_NSQ;
-            const uint32_t sQ1 = sQ0 + s1 * 2 * BWD_TILE;
+            const uint32_t sQ1 = q_at(jj + 1);
             if (j + 1 < ntot) {
               ok = mbar_wait(&bars[BB_Q_FULL + s1], ((jj + 1) / BWD_NSQ) & 1, abort_flag, p.status, BWD_CODE(3, BB_Q_FULL), p.bw.pipe_limit);
               if (!ok) break;
@@ -597,8 +695,13 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
               ok = mbar_wait(&bars[BB_DQ_FREE], jj & 1, abort_flag, p.status, BWD_CODE(3, BB_DQ_FREE), p.bw.pipe_limit);
               if (!ok) break;
               tc_fence_after();
+              if constexpr (BIAS) {
+                ok = mbar_wait(&bars[BB_DO_FULL], (jj + 1) & 1, abort_flag, p.status, BWD_CODE(3, BB_DO_FULL), p.bw.pipe_limit);
+                if (!ok) break;
+                tc_fence_after();
+              }
               BWD_TS(1, 5);
-              issue_st(tmem_base + TM_Y, sV, sQ1 + BWD_TILE);
+              issue_st(tmem_base + TM_Y, sV, do_at(jj + 1));
               tc_commit(&bars[BB_DP_FULL]);
               BWD_TS(1, 6);
             }
@@ -638,10 +741,14 @@ static int bwd_num_sms() {
 int launch_bwd_block(const lvx_shape& s, const void* q, const void* d_o, const float* lse, const float* delta,
                      const void* k, const void* v, const int32_t* kv_valid_len, float sm_scale, float* dq_acc,
                      float* dk_acc, float* dv_acc, int accumulate_dkdv, int* status, cudaStream_t st,
-                     const lvx_block_wait* bw) {
+                     const lvx_block_wait* bw, const lvx_bias* bias) {
   if (!(sm_scale > 0.f)) return fail(LVX_ERR_SHAPE, "lvx_bwd_block: sm_scale must be positive");
   if (accumulate_dkdv < 0 || accumulate_dkdv > 2)
     return fail(LVX_ERR_SHAPE, "lvx_bwd_block: accumulate_dkdv must be 0, 1 or 2 (got %d)", accumulate_dkdv);
+  // bias: the tensor-core form takes bf16 (see the head of this file)
+  if (bias && s.dtype != LVX_BF16)
+    return launch_bwd_block_simt(s, q, d_o, lse, delta, k, v, kv_valid_len, bias, sm_scale, dq_acc, dk_acc, dv_acc,
+                                 accumulate_dkdv, st);
   if (s.dtype == LVX_FP32)
     return launch_bwd_block_fp32(s, q, d_o, lse, delta, k, v, kv_valid_len, sm_scale, dq_acc, dk_acc, dv_acc,
                                  accumulate_dkdv, st);
@@ -675,6 +782,7 @@ int launch_bwd_block(const lvx_shape& s, const void* q, const void* d_o, const f
   p.accumulate = accumulate_dkdv;
   p.status = status;
   p.bw = make_block_wait(bw, qb);
+  p.bias = make_bias(s, bias);
 
   p.kv_tiles = (s.Skv + 127) / 128;
   p.nitems = p.kv_tiles * p.kv_slabs;
@@ -684,8 +792,9 @@ int launch_bwd_block(const lvx_shape& s, const void* q, const void* d_o, const f
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM);
     if (e == cudaSuccess) kern<<<grid, BWD_THREADS, BWD_SMEM, st>>>(tmQ, tmDO, tmK, tmV, p);
   };
-  if (s.dtype == LVX_BF16) go(bwd_kernel<true>);
-  else go(bwd_kernel<false>);
+  if (bias) go(bwd_kernel<true, true>);
+  else if (s.dtype == LVX_BF16) go(bwd_kernel<true, false>);
+  else go(bwd_kernel<false, false>);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(bwd)");
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "bwd_kernel launch");

@@ -66,13 +66,6 @@ __device__ __forceinline__ void load_tile(float* dst, const T* src, int row0, in
   }
 }
 
-// Dense additive bias on the scores: value for (query block, batch, query head, query row, key) at
-// base[blk*s_blk + b*s_b + h*s_h + i*s_q + j*s_kv] (strides in floats; 0 broadcasts). nullptr = no bias.
-struct BiasView {
-  const float* base;
-  long long s_blk, s_b, s_h, s_q, s_kv;
-  int sq, g;          // query rows per head, query heads per KV head (to unpack a packed row)
-};
 // pointer to the bias row of packed row `r` of query slab `slab` (kv slab `kvs`), or nullptr
 __device__ __forceinline__ const float* bias_row(const BiasView& b, int slab, int kvs, int kv_slabs, int hkv, int r) {
   if (b.base == nullptr) return nullptr;
@@ -387,19 +380,6 @@ fp32_bwd_kernel(const Fp32BwdParams p) {
       }
     }
   }
-}
-
-static BiasView make_bias(const lvx_shape& s, const lvx_bias* b) {
-  BiasView v;
-  v.base = b ? b->bias : nullptr;
-  v.s_blk = b ? b->stride_block : 0;
-  v.s_b = b ? b->stride_b : 0;
-  v.s_h = b ? b->stride_h : 0;
-  v.s_q = b ? b->stride_q : 0;
-  v.s_kv = b ? b->stride_kv : 0;
-  v.sq = s.Sq;
-  v.g = s.Hq / s.Hkv;
-  return v;
 }
 
 int launch_fwd_block_simt(const lvx_shape& s, const FwdPlan& pl, const void* q, const void* k, const void* v,

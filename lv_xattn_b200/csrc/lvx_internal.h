@@ -27,6 +27,26 @@ int validate_arch();
 inline int q_blocks_of(const lvx_shape& s) { return s.q_blocks > 1 ? s.q_blocks : 1; }
 inline int elt_size(int dtype) { return dtype == LVX_FP32 ? 4 : 2; }
 
+// Dense additive bias on the scores: value for (query block, batch, query head, query row, key) at
+// base[blk*s_blk + b*s_b + h*s_h + i*s_q + j*s_kv] (strides in floats; 0 broadcasts). nullptr = no bias.
+struct BiasView {
+  const float* base;
+  long long s_blk, s_b, s_h, s_q, s_kv;
+  int sq, g;          // query rows per head, query heads per KV head (to unpack a packed row)
+};
+inline BiasView make_bias(const lvx_shape& s, const lvx_bias* b) {
+  BiasView v;
+  v.base = b ? b->bias : nullptr;
+  v.s_blk = b ? b->stride_block : 0;
+  v.s_b = b ? b->stride_b : 0;
+  v.s_h = b ? b->stride_h : 0;
+  v.s_q = b ? b->stride_q : 0;
+  v.s_kv = b ? b->stride_kv : 0;
+  v.sq = s.Sq;
+  v.g = s.Hq / s.Hkv;
+  return v;
+}
+
 // Split-KV plan of the forward block; shared by the kernel launcher, the combine kernel and
 // lvx_query_workspace so that all three agree on the workspace layout.
 struct FwdPlan {
@@ -43,9 +63,8 @@ FwdPlan plan_fwd(const lvx_shape& s);
 // Launchers (one per .cu). `status` is the device status word.
 int launch_fwd_block(const lvx_shape& s, const FwdPlan& p, const void* q, const void* k, const void* v,
                      const int32_t* kv_valid_len, float sm_scale, float* o_part, float* ml_part, int* status,
-                     cudaStream_t st, const lvx_block_wait* bw = nullptr);
-// The forward block for few packed query rows (fwd_rows_sm100.cu); same plan and partials layout. Measured at one token
-// over 409,856 keys: 270 us a call against 447 with the 256-row kernel.
+                     cudaStream_t st, const lvx_block_wait* bw = nullptr, const lvx_bias* bias = nullptr);
+// The forward block for few packed query rows (fwd_rows_sm100.cu); same plan and partials layout.
 constexpr int kFewRows = 64;
 int launch_fwd_rows(const lvx_shape& s, const FwdPlan& p, const void* q, const void* k, const void* v,
                     const int32_t* kv_valid_len, float sm_scale, float* o_part, float* ml_part, int* status,
@@ -57,7 +76,7 @@ int launch_bwd_prep(const lvx_shape& s, const void* o, const void* d_o, float* d
 int launch_bwd_block(const lvx_shape& s, const void* q, const void* d_o, const float* lse, const float* delta,
                      const void* k, const void* v, const int32_t* kv_valid_len, float sm_scale, float* dq_acc,
                      float* dk_acc, float* dv_acc, int accumulate_dkdv, int* status, cudaStream_t st,
-                     const lvx_block_wait* bw = nullptr);
+                     const lvx_block_wait* bw = nullptr, const lvx_bias* bias = nullptr);
 // Limit of the in-kernel waits for a peer's flag, in SM cycles (lvx_p2p_set_timeout).
 long long p2p_wait_limit_cycles();
 // fp32 inputs (exact FP32-FMA kernels, same workspace layout and masking rules as the tensor-core path)

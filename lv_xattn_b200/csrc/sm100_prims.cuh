@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <stdint.h>
 
 namespace lvx {
@@ -326,6 +327,12 @@ __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
+}
+// The two values of a packed pair, exactly.
+template <bool IS_BF16>
+__device__ __forceinline__ float2 unpack16x2(uint32_t v) {
+  if (IS_BF16) return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+  return __half22float2(*reinterpret_cast<const __half2*>(&v));
 }
 // Two fp32 lanes per instruction (sm_100 packed arithmetic): halves the issue slots of the softmax inner loops.
 __device__ __forceinline__ uint64_t f32x2(float lo, float hi) {

@@ -128,7 +128,7 @@ def _block_wait(block_wait):
 
 def fwd_partials(q, k, v, sm_scale, kv_valid_len=None, bias=None, block_wait=None) -> FwdPartials:
     """Launches the forward block: Q block x local K/V shard -> split-KV partials in the workspace.
-    bias: optional dense additive fp32 bias on the scores (S = sm_scale*q.k + bias); runs the general kernels."""
+    bias: optional dense additive fp32 bias on the scores (S = sm_scale*q.k + bias)."""
     _require_cuda(q, k, v, kv_valid_len)
     lib = _lib.load()
     q, k, v = _contig(q), _contig(k), _contig(v)

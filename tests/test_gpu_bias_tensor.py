@@ -1,0 +1,89 @@
+"""The tensor-core form of the biased blocks: every stride and shape that its loads distinguish, masks of -inf and of the
+type's lowest value, rows without any key, and what its two-part P and dS keep of the fp32 values they stand for."""
+import math
+
+import pytest
+import torch
+
+import _parity
+from oracle import attention_oracle as orc
+
+pytestmark = pytest.mark.gpu
+SCALE = 1.0 / math.sqrt(128.0)
+
+
+def bias_of(kind, B, Hq, Sq, Skv, device):
+    g = torch.Generator().manual_seed(5)
+    if kind == "shared":                                   # one row per query, every head alike
+        return torch.randn(1, 1, Sq, Skv, generator=g).to(device)
+    if kind == "per_head":
+        return torch.randn(B, Hq, Sq, Skv, generator=g).to(device)
+    if kind == "keys":                                     # query stride 0
+        return torch.randn(B, 1, 1, Skv, generator=g).to(device)
+    if kind == "queries":                                  # key stride 0
+        return torch.randn(B, 1, Sq, 1, generator=g).to(device)
+    if kind == "transposed":                               # key stride > 1
+        return torch.randn(1, 1, Skv, Sq, generator=g).to(device).transpose(2, 3)
+    if kind == "offset":                                   # rows that start off a 16-byte boundary
+        return torch.randn(1, 1, Sq, Skv + 1, generator=g).to(device)[..., 1:]
+    b = torch.zeros(1, 1, Sq, Skv)
+    b[..., Skv // 3:] = torch.finfo(torch.float32).min if kind == "lowest" else float("-inf")
+    b[:, :, Sq // 2] = float("-inf")                       # a query that sees nothing
+    return b.to(device)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kind", ["shared", "per_head", "keys", "queries", "transposed", "offset", "lowest", "masked"])
+@pytest.mark.parametrize("shape", [(2, 4, 2, 77, 388), (1, 8, 1, 5, 129), (1, 2, 2, 300, 1024)])
+def test_bias_forms(cuda_device, shape, kind, dtype):
+    from lv_xattn_b200 import ops, _lib
+    B, Hq, Hkv, Sq, Skv = shape
+    q, k, v, do = orc.make_inputs(B, Hq, Hkv, Sq, Skv, 128, 71, dtype)
+    bias = bias_of(kind, B, Hq, Sq, Skv, cuda_device)
+    valid = [Skv - 3, Skv // 2][:B]
+    bias_ref, do_ref = bias.cpu().expand(B, bias.shape[1], Sq, Skv), do.clone()
+    if kind in ("lowest", "masked"):
+        # the oracle gets the query that sees nothing as one without a gradient; its output is zero and its lse -inf
+        bias_ref = bias_ref.clone()
+        bias_ref[:, :, Sq // 2] = 0
+        do_ref[:, :, Sq // 2] = 0
+    ref = orc.attention_fwd_bwd(q, k, v, do_ref, SCALE, valid, bias=bias_ref)
+    if kind in ("lowest", "masked"):
+        ref[0][:, :, Sq // 2] = 0
+        ref[1][:, :, Sq // 2] = float("-inf")
+    qd, kd, vd, dod = (t.to(cuda_device) for t in (q, k, v, do))
+    kvl = torch.tensor(valid, dtype=torch.int32, device=cuda_device)
+    o, lse = ops.fwd_block(qd, kd, vd, SCALE, kv_valid_len=kvl, bias=bias)
+    delta = ops.bwd_prep(o, dod)
+    dq = torch.zeros(B, Hq, Sq, 128, device=cuda_device)
+    dk, dv = torch.empty_like(kd), torch.empty_like(vd)
+    ops.bwd_block(qd, dod, lse, delta, kd, vd, SCALE, dq, dk, dv, "final", kvl, bias=bias)
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    label = f"bias_{kind}{shape}{dtype}"
+    _parity.assert_lse_close(lse.cpu().view(B, Hq, Sq), ref[1], label)
+    _parity.assert_close(o.float().cpu(), ref[0], "o", label, *_parity.BF16["o"])
+    _parity.assert_grads_16bit((dq, dk, dv), ref[2:], label)
+
+
+def test_two_part_operands(cuda_device):
+    """fp32 outputs against 64 bits. P and dS are held to 2^-17 of each value (two bf16 numbers), the scores to fp32 sums
+    over 128 products; 2^-15 leaves a factor of four. One bf16 rounding would show at 2^-9."""
+    from lv_xattn_b200 import ops
+    B, Hq, Hkv, Sq, Skv = 1, 4, 2, 160, 1000
+    q, k, v, do = orc.make_inputs(B, Hq, Hkv, Sq, Skv, 128, 73, torch.bfloat16)
+    bias = torch.randn(1, 1, Sq, Skv, generator=torch.Generator().manual_seed(74))
+    q6, k6, v6, do6 = (t.double().requires_grad_() for t in (q, k, v, do))
+    s = q6 @ k6.repeat_interleave(2, 1).transpose(-1, -2) * SCALE + bias.double()
+    o6 = s.softmax(-1) @ v6.repeat_interleave(2, 1)
+    dq6, dk6, dv6 = torch.autograd.grad(o6, (q6, k6, v6), do6)
+    d = cuda_device
+    qd, kd, vd, dod, bd = (t.to(d) for t in (q, k, v, do, bias))
+    o, lse = ops.fwd_block(qd, kd, vd, SCALE, final=False, bias=bd)
+    delta = (o6.detach() * do6.detach()).sum(-1).float().view(Hq, Sq).to(d)
+    dq = torch.zeros(B, Hq, Sq, 128, device=d)
+    dk, dv = torch.empty(B, Hkv, Skv, 128, device=d), torch.empty(B, Hkv, Skv, 128, device=d)
+    ops.bwd_block(qd, dod, lse, delta, kd, vd, SCALE, dq, dk, dv, False, bias=bd)
+    for name, got, ref in (("o", o, o6), ("dq", dq, dq6), ("dk", dk, dk6), ("dv", dv, dv6)):
+        err = ((got.cpu().double() - ref).norm() / ref.norm()).item()
+        assert err <= 2.0 ** -15, (name, err)
