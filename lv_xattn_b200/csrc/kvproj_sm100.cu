@@ -23,6 +23,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <math.h>
+#include <algorithm>
 
 namespace lvx {
 
@@ -305,67 +306,88 @@ int launch_kv_project(int dtype, const void* x, const void* wk, const void* wv, 
 // ---------------------------------------------------------------------------------------------
 // Backward of the fused norm: from dK (gradient of the normalised keys), K (normalised), rstd and w
 //   dKpre = rstd * (w * dK - (K / w) * mean_d(K * dK))          dw[d] += sum_rows dK * K / w
-// One warp per (key, head) row of 128; dw is reduced per block and added with one atomic per column and block.
+// Bound by memory: k and dk in, dKpre out, 768 bytes per (key, head) row. Half a warp works on a row (16 bytes a lane),
+// every half-warp has four rows in flight and walks on through the tensor with its share of dw in registers, so that a
+// block adds to dw once: with one block per eight rows and an atomic per column and block, the 128 addresses of dw were
+// what the kernel waited for. Measured on 8 heads x 51,232 keys (315 MB): 235 -> 68 us.
+constexpr int KN_ROWS = 4;              // rows in flight per half-warp
+constexpr int KN_BLOCK_ROWS = 16 * KN_ROWS;
+
 template <bool IS_BF16>
 __global__ void __launch_bounds__(256)
 knorm_bwd_kernel(const void* __restrict__ k, const void* __restrict__ dk, const float* __restrict__ rstd,
                  const void* __restrict__ norm_w, void* __restrict__ dkpre, float* __restrict__ dw, long rows,
                  const int* status) {
   if (status && *reinterpret_cast<const volatile int*>(status) != 0) return;
-  __shared__ float s_dw[8][128];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const long row = long(blockIdx.x) * 8 + wib;
-  float dwl[4] = {0.f, 0.f, 0.f, 0.f};
-  if (row < rows) {
-    const uint2 kk = reinterpret_cast<const uint2*>(k)[row * 32 + lane];
-    const uint2 gg = reinterpret_cast<const uint2*>(dk)[row * 32 + lane];
-    const uint2 ww = reinterpret_cast<const uint2*>(norm_w)[lane];
-    float kf[4], gf[4], wf[4];
-    auto unpack = [](uint32_t v, float& a, float& b) {
-      if (IS_BF16) {
-        a = __uint_as_float(v << 16);
-        b = __uint_as_float(v & 0xffff0000u);
-      } else {
-        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
-        a = f.x;
-        b = f.y;
-      }
-    };
-    unpack(kk.x, kf[0], kf[1]);
-    unpack(kk.y, kf[2], kf[3]);
-    unpack(gg.x, gf[0], gf[1]);
-    unpack(gg.y, gf[2], gf[3]);
-    unpack(ww.x, wf[0], wf[1]);
-    unpack(ww.y, wf[2], wf[3]);
-    float dot = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dot = fmaf(kf[i], gf[i], dot);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off);
-    const float mean = dot * (1.f / 128.f), r = rstd[row];
-    float o[4];
+  __shared__ float s_dw[16][128];
+  const int half = threadIdx.x >> 4, l16 = threadIdx.x & 15;      // half-warp of the block, lane in it: columns 8*l16..
+  auto unpack8 = [](const uint4& v, float (&f)[8]) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float xhat = kf[i] / wf[i];                // Kpre * rstd
-      o[i] = r * (wf[i] * gf[i] - xhat * mean);
-      dwl[i] = gf[i] * xhat;
+      const float2 t = unpack16x2<IS_BF16>(w[i]);
+      f[2 * i] = t.x;
+      f[2 * i + 1] = t.y;
     }
-    reinterpret_cast<uint2*>(dkpre)[row * 32 + lane] = make_uint2(kp_pack<IS_BF16>(o[0], o[1]), kp_pack<IS_BF16>(o[2], o[3]));
+  };
+  float wf[8], dwl[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {      // norm_w is 8-byte aligned
+    const float2 t = unpack16x2<IS_BF16>(reinterpret_cast<const uint32_t*>(norm_w)[l16 * 4 + i]);
+    wf[2 * i] = t.x;
+    wf[2 * i + 1] = t.y;
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) s_dw[wib][lane * 4 + i] = dwl[i];
+  for (int i = 0; i < 8; ++i) dwl[i] = 0.f;
+  for (long base = long(blockIdx.x) * KN_BLOCK_ROWS; base < rows; base += long(gridDim.x) * KN_BLOCK_ROWS) {
+    uint4 kk[KN_ROWS], gg[KN_ROWS];
+    float rs[KN_ROWS];
+#pragma unroll
+    for (int u = 0; u < KN_ROWS; ++u) {
+      const long row = min(base + u * 16 + half, rows - 1);
+      kk[u] = reinterpret_cast<const uint4*>(k)[row * 16 + l16];
+      gg[u] = reinterpret_cast<const uint4*>(dk)[row * 16 + l16];
+      rs[u] = rstd[row];
+    }
+#pragma unroll
+    for (int u = 0; u < KN_ROWS; ++u) {
+      const long row = base + u * 16 + half;
+      float kf[8], gf[8];
+      unpack8(kk[u], kf);
+      unpack8(gg[u], gf);
+      float dot = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) dot = fmaf(kf[i], gf[i], dot);
+#pragma unroll
+      for (int off = 8; off > 0; off >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off);
+      if (row >= rows) continue;
+      const float mean = dot * (1.f / 128.f), r = rs[u];
+      float o[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float xhat = kf[i] / wf[i];                // Kpre * rstd
+        o[i] = r * (wf[i] * gf[i] - xhat * mean);
+        dwl[i] = fmaf(gf[i], xhat, dwl[i]);
+      }
+      reinterpret_cast<uint4*>(dkpre)[row * 16 + l16] =
+          make_uint4(kp_pack<IS_BF16>(o[0], o[1]), kp_pack<IS_BF16>(o[2], o[3]), kp_pack<IS_BF16>(o[4], o[5]),
+                     kp_pack<IS_BF16>(o[6], o[7]));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) s_dw[half][l16 * 8 + i] = dwl[i];
   __syncthreads();
   if (threadIdx.x < 128) {
     float a = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) a += s_dw[w][threadIdx.x];
+    for (int w = 0; w < 16; ++w) a += s_dw[w][threadIdx.x];
     atomicAdd(dw + threadIdx.x, a);
   }
 }
 
 int launch_knorm_bwd(int dtype, const void* k, const void* dk, const float* rstd, const void* norm_w, void* dkpre,
                      float* dw, long rows, cudaStream_t st) {
-  const long blocks = (rows + 7) / 8;
+  const long blocks = std::min<long>((rows + KN_BLOCK_ROWS - 1) / KN_BLOCK_ROWS, 148 * 6);
   if (blocks == 0) return LVX_OK;
   const int* sp = device_status_ptr();
   if (dtype == LVX_BF16) knorm_bwd_kernel<true><<<blocks, 256, 0, st>>>(k, dk, rstd, norm_w, dkpre, dw, rows, sp);
