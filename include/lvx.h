@@ -77,6 +77,17 @@ int lvx_device_status(void* stream, int* status_out);
  * without synchronising; the reference would simply block for ever (lv_xattn/async_communication.py:301-305). */
 int lvx_device_status_peek(void* stream, int* host_out);
 
+/* The host's own copy of the current device's word: *host_word points to an int that lvx_fwd_combine_merge and
+ * lvx_add_cast (the last kernels of a forward and a backward) write when they find the word set (mapped pinned memory, kept
+ * for the life of the process, cleared by lvx_device_status), so that a host loop can look at it before every call at the
+ * price of a memory read. Set up by the first call; NULL if that call comes while `stream`
+ * is being captured. No reference counterpart (its waits are unbounded, lv_xattn/async_communication.py:301-305). */
+int lvx_device_status_host(void* stream, const int** host_word);
+
+/* Global key-padding lengths -> this rank's: out[i] = clamp(valid_len[i] - first_key, 0, skv) for `count` host values,
+ * which travel as kernel arguments (no copy, no synchronisation). The reference has no key padding of its own. */
+int lvx_local_valid(const int64_t* valid_len, int count, int64_t first_key, int skv, int32_t* out, void* stream);
+
 /* Bytes of scratch the forward / backward block kernels need for this shape.
  * Stands in for the per-step torch allocations in lv_xattn/attn.py:382-385 and
  * lv_xattn/flash_attn_kernels.py:920-921. */
@@ -141,6 +152,18 @@ int lvx_fwd_block_bias(const lvx_shape* s, const void* q, const void* k, const v
 int lvx_bwd_block_bias(const lvx_shape* s, const void* q, const void* d_o, const float* lse, const float* delta,
                        const void* k, const void* v, const int32_t* kv_valid_len, const lvx_bias* bias,
                        float sm_scale, float* dq_acc, void* dk_acc, void* dv_acc, int accumulate_dkdv, void* stream);
+
+/* The whole attention of one query block against the resident K/V, with nothing travelling: lvx_fwd_block (or its
+ * _bias form when `bias` is given) and the combine in one call, and lvx_bwd_prep, the cleared dQ accumulator, the
+ * backward block and the cast of dQ in one call. Same arguments and results as the calls they stand for; `scratch` of the
+ * backward holds 4*(128+1)*q_blocks*B*Hq*Sq bytes (fp32 dQ, then delta). These are the W = 1 body of
+ * lv_xattn/attn.py:297-435 and :437-545. */
+int lvx_attn_forward(const lvx_shape* s, const void* q, const void* k, const void* v, const int32_t* kv_valid_len,
+                     const lvx_bias* bias, float sm_scale, void* workspace, size_t workspace_bytes, void* o,
+                     float* lse, void* stream);
+int lvx_attn_backward(const lvx_shape* s, const void* d_o, const void* q, const void* k, const void* v, const void* o,
+                      const float* lse, const int32_t* kv_valid_len, const lvx_bias* bias, float sm_scale,
+                      void* scratch, size_t scratch_bytes, void* dq, void* dk, void* dv, void* stream);
 
 /* K/V projection of the visual states with the per-head RMSNorm of K fused in: one tensor-core GEMM
  *   Kpre = X Wk^T, V = X Wv^T,   K = Kpre * rsqrt(mean_d(Kpre^2) + eps) * norm_w   (per key and head, d = 0..127)

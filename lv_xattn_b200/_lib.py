@@ -22,6 +22,7 @@ SYMBOLS = [
     "lvx_query_workspace", "lvx_fwd_block", "lvx_fwd_block_bias", "lvx_bwd_block_bias",
     "lvx_kv_project", "lvx_knorm_bwd", "lvx_fwd_block_gathered", "lvx_bwd_block_gathered",
     "lvx_fwd_combine_merge", "lvx_bwd_prep", "lvx_bwd_block", "lvx_add_cast", "lvx_selftest_mma",
+    "lvx_attn_forward", "lvx_attn_backward", "lvx_local_valid", "lvx_device_status_host",
     "lvx_fwd_block_static", "lvx_fwd_merge_parts", "lvx_sum_cast",
     "lvx_p2p_signal", "lvx_p2p_gather", "lvx_p2p_fwd_merge", "lvx_p2p_sum_cast", "lvx_p2p_push", "lvx_p2p_wait",
     "lvx_p2p_push_dma",
@@ -99,6 +100,10 @@ def load():
     lib.lvx_fwd_merge_parts.argtypes = [sp, fp, fp, ctypes.c_int, ctypes.c_size_t, ctypes.c_size_t, vp, fp, vp]
     lib.lvx_sum_cast.argtypes = [fp, ctypes.c_int, ctypes.c_size_t, vp, ctypes.c_int, ctypes.c_size_t, vp]
     lib.lvx_fwd_block_static.argtypes = [sp, vp, vp, vp, i32p, ctypes.c_float, vp, fp, vp]
+    lib.lvx_attn_forward.argtypes = [sp, vp, vp, vp, i32p, bp, ctypes.c_float, vp, ctypes.c_size_t, vp, fp, vp]
+    lib.lvx_attn_backward.argtypes = [sp, vp, vp, vp, vp, vp, fp, i32p, bp, ctypes.c_float, vp, ctypes.c_size_t, vp, vp, vp, vp]
+    lib.lvx_local_valid.argtypes = [vp, ctypes.c_int, ctypes.c_int64, ctypes.c_int, i32p, vp]
+    lib.lvx_device_status_host.argtypes = [vp, ctypes.POINTER(ctypes.c_void_p)]
     for name in SYMBOLS:
         getattr(lib, name)  # AttributeError here means header and library disagree
         if name != "lvx_last_error":
@@ -117,8 +122,18 @@ def ptr(t):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
 
+# torch.cuda.current_stream() builds a Stream object, at several times the price of the handle that is wanted of it
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def stream_int() -> int:
+    if _raw_stream is not None:
+        return _raw_stream(torch.cuda.current_device())
+    return torch.cuda.current_stream().cuda_stream
+
+
 def stream_ptr():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(stream_int())
 
 
 def make_shape(B, Hq, Hkv, Sq, Skv, D, dtype, q_blocks=1) -> LvxShape:
@@ -135,6 +150,14 @@ def query_workspace(shape: LvxShape):
     f, b = ctypes.c_size_t(0), ctypes.c_size_t(0)
     check(load().lvx_query_workspace(ctypes.byref(shape), ctypes.byref(f), ctypes.byref(b)), "lvx_query_workspace")
     return f.value, b.value
+
+
+def device_status_host():
+    """The current device's host copy of the status word as a ctypes int, or None while there is none (the current
+    stream is being captured)."""
+    p = ctypes.c_void_p()
+    check(load().lvx_device_status_host(stream_ptr(), ctypes.byref(p)), "lvx_device_status_host")
+    return ctypes.c_int.from_address(p.value) if p.value else None
 
 
 def device_status() -> int:

@@ -110,6 +110,11 @@ def _local_valid(kv_valid_len, skv_local: int, device):
     """Global key-padding lengths [B] -> this rank's clamp min(max(valid - rank*Skv_l, 0), Skv_l)."""
     if kv_valid_len is None:
         return None
+    if device.type == "cuda":
+        host = torch.as_tensor(kv_valid_len)
+        if not host.is_cuda:       # a list, or a tensor in host memory: no copy to wait for
+            return ops.local_valid(host.to(torch.int64).contiguous(), get_sequence_parallel_rank() * skv_local, skv_local,
+                                   device)
     t = torch.as_tensor(kv_valid_len, device=device).to(torch.int64)
     t = (t - get_sequence_parallel_rank() * skv_local).clamp_(0, skv_local)
     return t.to(torch.int32).contiguous()
@@ -142,6 +147,17 @@ def _status_post(t):
         status_watch.post()
 
 
+def _one_call(q, W):
+    """True for a call on one GPU without a group: each pass is then a single library call (ops.attn_forward /
+    attn_backward), and a wait that ran out in an earlier call is noticed here through the host's copy of the status word.
+    While ops records kernel times the step loop's own calls are used, which it knows how to time."""
+    if W != 1 or not q.is_cuda or ops.profiling():
+        return False
+    from .peer_memory import status_watch
+    status_watch.watch(q.device.index)
+    return True
+
+
 def _carve(buf: torch.Tensor, offset: int, shape, dtype) -> torch.Tensor:
     n = 1
     for s in shape:
@@ -158,8 +174,10 @@ def _attn_forward(q, k, v, causal, sm_scale, comm_mode, bias_func=None, local_bi
     reference :294-296); the result is then the attention of the local Q block over the local K/V only.
     kv_valid_len: optional global number of valid K/V rows per batch entry (key padding)."""
     _check_common(q, k, v, causal, bias_func, local_bias_args, remote_bias_args)
-    _status_poll(q)
     W = get_sequence_parallel_size()
+    local = _one_call(q, W)
+    if not local:
+        _status_poll(q)
     B, Hq, Sq, D = q.shape
     dev, dt = q.device, q.dtype
     es = q.element_size()
@@ -168,6 +186,10 @@ def _attn_forward(q, k, v, causal, sm_scale, comm_mode, bias_func=None, local_bi
     o = torch.empty(B, Hq, Sq, D, dtype=dt, device=dev)
     L = torch.empty(B * Hq, Sq, dtype=torch.float32, device=dev)
 
+    if local:
+        bias = _build_bias(bias_func, local_bias_args, remote_bias_args, qc, kc)
+        ops.attn_forward(qc, kc, vc, sm_scale, kvl, bias, o, L)
+        return q, k, v, o, L
     if W == 1 or comm_mode == "nocomm":
         bias = _build_bias(bias_func, local_bias_args, remote_bias_args, qc, kc)
         for _ in range(W):
@@ -341,8 +363,10 @@ def _attn_backward(do, q, k, v, o, L, causal, sm_scale, comm_mode, backward_engi
     """Returns (dq, dk, dv): dq like q, dk/dv like k/v (summed over the query heads of each KV group)
     (reference :437-545). `backward_engine` is accepted and ignored, as in the reference."""
     _check_common(q, k, v, causal, bias_func, local_bias_args, remote_bias_args)
-    _status_poll(q)
     W = get_sequence_parallel_size()
+    local = _one_call(q, W)
+    if not local:
+        _status_poll(q)
     B, Hq, Sq, D = q.shape
     Hkv, Skv = k.shape[1], k.shape[2]
     dev, dt = q.device, q.dtype
@@ -354,6 +378,14 @@ def _attn_backward(do, q, k, v, o, L, causal, sm_scale, comm_mode, backward_engi
     kvl = _local_valid(kv_valid_len, Skv, dev)
 
     n_q, n_r, n_kv = B * Hq * Sq * D, B * Hq * Sq, B * Hkv * Skv * D
+    if local:
+        dq = torch.empty(B, Hq, Sq, D, dtype=dt, device=dev)
+        dk = torch.empty(B, Hkv, Skv, D, dtype=dt, device=dev)
+        dv = torch.empty(B, Hkv, Skv, D, dtype=dt, device=dev)
+        bias = _build_bias(bias_func, local_bias_args, remote_bias_args, qc, kc)
+        scratch = get_slabs("bwd_dq_delta", (n_q + n_r) * 4, dev, 1)[0]
+        ops.attn_backward(doc, qc, kc, vc, oc, Lc, sm_scale, kvl, bias, scratch, dq, dk, dv)
+        return dq, dk, dv
     delta = ops.bwd_prep(oc, doc)                       # once, at home; travels instead of O
     dq = torch.empty(B, Hq, Sq, D, dtype=dt, device=dev)
 

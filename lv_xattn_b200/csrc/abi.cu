@@ -4,6 +4,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 namespace lvx {
 
@@ -22,8 +23,9 @@ int cuda_fail(cudaError_t e, const char* what) {
   return static_cast<int>(e) > 0 ? static_cast<int>(e) : 1;
 }
 
-// Device status word: one per device that loads the library, written by bounded waits that ran out.
-__device__ int g_status_word[4];
+// Device status word: one per device that loads the library, written by bounded waits that ran out. Words 2-3 hold the
+// address of the host's copy (publish_status in elementwise.cu), once there is one.
+__device__ __align__(16) int g_status_word[4];
 
 static int* status_ptr() {
   static int* ptrs[64] = {};
@@ -35,6 +37,30 @@ static int* status_ptr() {
     ptrs[dev] = static_cast<int*>(p);
   }
   return ptrs[dev];
+}
+
+// The host's copy of the current device's status word: mapped pinned memory, set up by the first call that asks for it
+// and kept for the process. nullptr while `st` is being captured and there is none yet (its set-up is not capturable).
+static int* g_host_status[64];
+static int* host_status_word(cudaStream_t st) {
+  static std::mutex mu;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (g_host_status[dev]) return g_host_status[dev];
+  int* sp = status_ptr();
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (!sp || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return nullptr;
+  void *h = nullptr, *d = nullptr;
+  if (cudaHostAlloc(&h, 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+  *static_cast<volatile int*>(h) = 0;
+  if (cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess ||
+      cudaMemcpy(sp + 2, &d, sizeof(d), cudaMemcpyHostToDevice) != cudaSuccess) {
+    cudaFreeHost(h);
+    return nullptr;
+  }
+  g_host_status[dev] = static_cast<int*>(h);
+  return g_host_status[dev];
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -139,6 +165,44 @@ int lvx_device_status(void* stream, int* status_out) {
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(status)");
   e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize(status)");
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && g_host_status[dev])
+    *reinterpret_cast<volatile int*>(g_host_status[dev]) = 0;
+  return LVX_OK;
+}
+
+int lvx_device_status_host(void* stream, const int** host_word) {
+  if (!host_word) return fail(LVX_ERR_NULL, "lvx_device_status_host: host_word is NULL");
+  *host_word = host_status_word(static_cast<cudaStream_t>(stream));
+  return LVX_OK;
+}
+
+// Key-padding lengths given by the host, handed to the kernel by value: no copy, no synchronisation, capturable.
+struct ValidLens {
+  int64_t v[256];
+};
+__global__ void local_valid_kernel(const __grid_constant__ ValidLens lens, int n, int64_t base, int skv, int32_t* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int64_t left = lens.v[i] - base;
+  out[i] = int32_t(left < 0 ? 0 : left > skv ? skv : left);
+}
+
+int lvx_local_valid(const int64_t* valid_len, int count, int64_t first_key, int skv, int32_t* out, void* stream) {
+  const char* who = "lvx_local_valid";
+  if (count < 0 || skv < 0) return fail(LVX_ERR_SHAPE, "%s: negative count or skv", who);
+  if (count == 0) return LVX_OK;
+  if (!valid_len) return fail(LVX_ERR_NULL, "%s: valid_len is NULL", who);
+  LVX_REQUIRE_PTR(out, who);
+  for (int i0 = 0; i0 < count; i0 += 256) {
+    ValidLens lens;
+    const int n = count - i0 < 256 ? count - i0 : 256;
+    memset(&lens, 0, sizeof(lens));
+    memcpy(lens.v, valid_len + i0, size_t(n) * sizeof(int64_t));
+    local_valid_kernel<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(lens, n, first_key, skv, out + i0);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "local_valid launch");
+  }
   return LVX_OK;
 }
 
@@ -317,6 +381,43 @@ int lvx_bwd_block_bias(const lvx_shape* s, const void* q, const void* d_o, const
   if (!sp) return fail(LVX_ERR_DRIVER, "%s: status word unavailable", who);
   return launch_bwd_block(*s, q, d_o, lse, delta, k, v, kv_valid_len, sm_scale, dq_acc, static_cast<float*>(dk_acc),
                           static_cast<float*>(dv_acc), accumulate_dkdv, sp, static_cast<cudaStream_t>(stream), nullptr, bias);
+}
+
+int lvx_attn_forward(const lvx_shape* s, const void* q, const void* k, const void* v, const int32_t* kv_valid_len,
+                     const lvx_bias* bias, float sm_scale, void* workspace, size_t workspace_bytes, void* o, float* lse,
+                     void* stream) {
+  const int rc = bias ? lvx_fwd_block_bias(s, q, k, v, kv_valid_len, bias, sm_scale, workspace, workspace_bytes, stream)
+                      : lvx_fwd_block(s, q, k, v, kv_valid_len, sm_scale, workspace, workspace_bytes, stream);
+  return rc ? rc : lvx_fwd_combine_merge(s, workspace, nullptr, nullptr, o, lse, 1, stream);
+}
+
+int lvx_attn_backward(const lvx_shape* s, const void* d_o, const void* q, const void* k, const void* v, const void* o,
+                      const float* lse, const int32_t* kv_valid_len, const lvx_bias* bias, float sm_scale, void* scratch,
+                      size_t scratch_bytes, void* dq, void* dk, void* dv, void* stream) {
+  const char* who = "lvx_attn_backward";
+  int rc = check_shape(s, who);
+  if (rc) return rc;
+  LVX_REQUIRE_PTR(o, who);
+  LVX_REQUIRE_PTR(d_o, who);
+  LVX_REQUIRE_PTR(dq, who);
+  LVX_REQUIRE_PTR(scratch, who);
+  const size_t rows = size_t(q_blocks_of(*s)) * s->B * s->Hq * s->Sq, n_q = rows * 128;
+  if (scratch_bytes < n_q * sizeof(float) + rows * sizeof(float))
+    return fail(LVX_ERR_WORKSPACE, "%s: scratch has %zu bytes, %zu needed", who, scratch_bytes,
+                n_q * sizeof(float) + rows * sizeof(float));
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // fp32: dQ is accumulated where it is wanted; otherwise in the scratch, and cast at the end
+  const bool direct = s->dtype == LVX_FP32;
+  float* dq_acc = direct ? static_cast<float*>(dq) : static_cast<float*>(scratch);
+  float* delta = static_cast<float*>(scratch) + n_q;
+  if ((rc = launch_bwd_prep(*s, o, d_o, delta, st))) return rc;
+  const cudaError_t e = cudaMemsetAsync(dq_acc, 0, n_q * sizeof(float), st);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(dq)");
+  rc = bias ? lvx_bwd_block_bias(s, q, d_o, lse, delta, k, v, kv_valid_len, bias, sm_scale, dq_acc, dk, dv, 2, stream)
+            : lvx_bwd_block(s, q, d_o, lse, delta, k, v, kv_valid_len, sm_scale, dq_acc, static_cast<float*>(dk),
+                            static_cast<float*>(dv), 2, nullptr, 0, stream);
+  if (rc || direct) return rc;
+  return launch_add_cast(dq_acc, nullptr, dq, s->dtype, n_q, st);
 }
 
 int lvx_kv_project(int dtype, const void* x, const void* wk, const void* wv, const void* norm_w, float eps, int batch,

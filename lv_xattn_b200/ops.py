@@ -21,6 +21,10 @@ def set_profiling(on: bool) -> None:
     _profile = {"fwd": [], "bwd": [], "proj": []} if on else None
 
 
+def profiling() -> bool:
+    return _profile is not None
+
+
 def take_profile():
     """Returns {"fwd": [ms, ...], "bwd": [ms, ...]} for the launches since set_profiling(True); the caller
     must have synchronised the device."""
@@ -192,6 +196,64 @@ def fwd_block(q, k, v, sm_scale, kv_valid_len=None, o_in=None, lse_in=None, fina
     lse_out = torch.empty(q.numel() // (Hq * Sq * q.shape[-1]) * Hq, Sq, dtype=torch.float32, device=q.device)
     fwd_combine(part, o_in, lse_in, o_out, lse_out, final)
     return o_out, lse_out
+
+
+_fwd_bytes: dict = {}      # lvx_query_workspace is a function of the sizes alone
+
+
+def attn_forward(q, k, v, sm_scale, kv_valid_len, bias, o, lse) -> None:
+    """The whole attention of a [B, Hq, Sq, D] block against the local K/V in one library call (block and combine):
+    o like q, lse fp32 [B*Hq, Sq]. q, k, v are contiguous and checked by the caller."""
+    _require_cuda(q, k, v, kv_valid_len)
+    lib = _lib.load()
+    if v.shape != k.shape:
+        raise ValueError("k and v must have the same shape, and q/k/v the same dtype")
+    shp = shape_of(q, k)
+    key = (shp.B, shp.Hq, shp.Hkv, shp.Sq, shp.Skv, shp.dtype)
+    nbytes = _fwd_bytes.get(key)
+    if nbytes is None:
+        if len(_fwd_bytes) >= 4096:
+            _fwd_bytes.clear()
+        nbytes = _fwd_bytes[key] = _lib.query_workspace(shp)[0]
+    ws = _workspace(q.device, nbytes)
+    if kv_valid_len is not None and kv_valid_len.numel() != shp.B:
+        raise ValueError("kv_valid_len must be an int32 tensor with one entry per batch element")
+    bv, keep = _bias_view(bias, q, k) if bias is not None else (None, None)
+    _lib.check(lib.lvx_attn_forward(ctypes.byref(shp), q.data_ptr(), k.data_ptr(), v.data_ptr(),
+                                    None if kv_valid_len is None else kv_valid_len.data_ptr(),
+                                    None if bv is None else ctypes.byref(bv), float(sm_scale), ws.data_ptr(), ws.numel(),
+                                    o.data_ptr(), lse.data_ptr(), _lib.stream_int()), "lvx_attn_forward")
+    _count(2)
+
+
+def attn_backward(do, q, k, v, o, lse, sm_scale, kv_valid_len, bias, scratch, dq, dk, dv) -> None:
+    """Its backward in one library call: delta, the cleared dQ accumulator (both in `scratch`, uint8), the block, and dQ
+    cast to its dtype. All tensors contiguous and checked by the caller."""
+    _require_cuda(do, q, k, v, o, lse, kv_valid_len)
+    lib = _lib.load()
+    if v.shape != k.shape or do.numel() != q.numel() or o.numel() != q.numel() or do.dtype != q.dtype or o.dtype != q.dtype:
+        raise ValueError("do and o must be like q, and v like k")
+    shp = shape_of(q, k)
+    if kv_valid_len is not None and kv_valid_len.numel() != shp.B:
+        raise ValueError("kv_valid_len must be an int32 tensor with one entry per batch element")
+    bv, keep = _bias_view(bias, q, k) if bias is not None else (None, None)
+    _lib.check(lib.lvx_attn_backward(ctypes.byref(shp), do.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(),
+                                     o.data_ptr(), lse.data_ptr(), None if kv_valid_len is None else kv_valid_len.data_ptr(),
+                                     None if bv is None else ctypes.byref(bv), float(sm_scale), scratch.data_ptr(),
+                                     scratch.numel(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _lib.stream_int()),
+               "lvx_attn_backward")
+    _count(2 if q.dtype == torch.float32 else 3)
+
+
+def local_valid(valid_len, first_key: int, skv: int, device):
+    """clamp(valid_len - first_key, 0, skv) as int32 on the device, from a host tensor of int64 lengths. The values travel
+    as kernel arguments, so the host neither copies nor waits."""
+    out = torch.empty(valid_len.shape, dtype=torch.int32, device=device)
+    n = valid_len.numel()
+    _lib.check(_lib.load().lvx_local_valid(valid_len.data_ptr(), n, first_key, skv, out.data_ptr(),
+                                           _lib.stream_int()), "lvx_local_valid")
+    _count()
+    return out
 
 
 def bwd_prep(o, do):

@@ -127,6 +127,20 @@ class StatusWatch:
     def __init__(self):
         self._slots = []          # [pinned int32 tensor, event or None]
         self._next = 0
+        self._words = {}          # device index -> the host's copy of its status word (ctypes int)
+
+    def watch(self, device_index):
+        """Start of a call that exchanges nothing: such calls post no copies. The library keeps a copy of the status word
+        in host memory, which the last kernel of a pass writes when it finds the word set; it is read here before the
+        call, and by check()."""
+        word = self._words.get(device_index)
+        if word is None:
+            word = _lib.device_status_host()
+            if word is None:
+                return
+            self._words[device_index] = word
+        if word.value:
+            self._raise(word.value)
 
     def _slot(self):
         if len(self._slots) < 4:
@@ -144,10 +158,13 @@ class StatusWatch:
         ev.synchronize()
         code = int(s[0].item())
         if code:
-            _lib.device_status()                      # clears the word (and synchronises)
-            from .async_communication import P2PTimeoutError
-            what = f"rank {code & 0xFF} did not signal within the limit" if (code & 0xFF00) == 0x1300 else "a pipeline wait ran out"
-            raise P2PTimeoutError(f"device status word {code:#x}: {what}; the results of the affected call are invalid")
+            self._raise(code)
+
+    def _raise(self, code):
+        _lib.device_status()                      # clears the word and its host copy (and synchronises)
+        from .async_communication import P2PTimeoutError
+        what = f"rank {code & 0xFF} did not signal within the limit" if (code & 0xFF00) == 0x1300 else "a pipeline wait ran out"
+        raise P2PTimeoutError(f"device status word {code:#x}: {what}; the results of the affected call are invalid")
 
     def post(self):
         s = self._slot()
@@ -164,10 +181,16 @@ class StatusWatch:
                 self._read(s)
 
     def check(self):
-        """Blocks until every posted copy has arrived and raises if any is non-zero."""
+        """Blocks until every posted copy has arrived, and until the devices watched without copies have finished what was
+        queued; raises if anything is non-zero."""
         for s in self._slots:
             if s[1] is not None:
                 self._read(s)
+        for index, word in self._words.items():
+            with torch.cuda.device(index):
+                torch.cuda.synchronize()
+                if word.value:
+                    self._raise(word.value)
 
 
 status_watch = StatusWatch()
