@@ -7,7 +7,7 @@ Workloads (N = 1..8 ranks, total work fixed => strong scaling; Q/dO and K/V are 
 the ranks, rank r takes the r-th slice, reference test.py:164-178; inputs are seeded synthetic tensors with the
 reference benchmark's distributions, test.py:101-107: q,k,v ~ N(0,0.5^2), dO ~ N(0,1)):
   config 2 (default, the headline)  B=1, Hq=32, Hkv=8, D=128, Sq=2048 text queries, Skv=131072 visual keys, bf16
-  config 1  the reference's CPU-runnable correctness shape: Sq=512, Skv=8192, fp32 (exact FP32-FMA kernels)
+  config 1  the reference's CPU-runnable correctness shape: Sq=512, Skv=8192, fp32 (tf32 products in three parts, fp32 sums)
   config 5  long-visual stress: B=2, Sq=256, Skv=1048576, key padding to 1048576 / 786432 valid keys, bf16
   config 4  end-to-end training step (forward, loss, backward, gradient all-reduce; no optimizer, as in the reference's
             driver test_llama3.py:710-737) of a random-init Llama-3.2-11B-Vision-shaped text decoder: 40 layers, gated
@@ -799,7 +799,7 @@ def main():
                 "hbm_gbs": alg_bytes / (ms_per_step * 1e-3) / 1e9, "hbm_peak_gbs": pk["hbm_gbs"],
                 "launches_per_step": {"fwd": len(prof["fwd"]) // args.steps, "bwd": len(prof["bwd"]) // args.steps}}
     if dtype == torch.float32:
-        roofline["note"] = ("fp32 inputs run the exact FP32-FMA kernels (correctness configuration); the fraction is "
+        roofline["note"] = ("fp32 inputs run the general kernels, three tf32 products for each (correctness configuration); the fraction is "
                             "quoted against the bf16 tensor peak for comparability and is expected to be small")
 
     # ---- parity probe (outside every timed region) --------------------------------------------------

@@ -29,7 +29,7 @@ extern "C" {
 
 #define LVX_ABI_VERSION 1
 
-enum lvx_dtype { LVX_BF16 = 0, LVX_FP16 = 1, LVX_FP32 = 2 /* exact fp32 on the FP32-FMA pipe, no TF32 */ };
+enum lvx_dtype { LVX_BF16 = 0, LVX_FP16 = 1, LVX_FP32 = 2 /* fp32 accuracy: products in three tf32 parts, fp32 sums */ };
 
 enum lvx_error {
   LVX_OK = 0,

@@ -46,7 +46,7 @@
 // columns, low halves in the rest) and dS^T takes two shared-memory tiles, which leaves one buffer for dO instead of
 // two (dO of tile j is free after dV(j), so its successor still arrives under the dS^T half). dV, dK and dQ^T take
 // 16 MMAs instead of 8. The transposed frame suits the bias: a warp's lanes are 32 consecutive keys, so a column's bias
-// values are one 128-byte read. fp16 stays with the FP32-FMA kernel: dS has no bound there, and half of it could
+// values are one 128-byte read. fp16 stays with the general kernel: dS has no bound there, and half of it could
 // fall among fp16's subnormals. Measured at 32 heads, 512 x 6,404: 436 us, 5,177 on the FP32-FMA kernel.
 #include "lvx_internal.h"
 #include "sm100_prims.cuh"
@@ -747,7 +747,7 @@ int launch_bwd_block(const lvx_shape& s, const void* q, const void* d_o, const f
     return fail(LVX_ERR_SHAPE, "lvx_bwd_block: accumulate_dkdv must be 0, 1 or 2 (got %d)", accumulate_dkdv);
   // bias: the tensor-core form takes bf16 (see the head of this file)
   if (bias && s.dtype != LVX_BF16)
-    return launch_bwd_block_simt(s, q, d_o, lse, delta, k, v, kv_valid_len, bias, sm_scale, dq_acc, dk_acc, dv_acc,
+    return launch_bwd_block_general(s, q, d_o, lse, delta, k, v, kv_valid_len, bias, sm_scale, dq_acc, dk_acc, dv_acc,
                                  accumulate_dkdv, st);
   if (s.dtype == LVX_FP32)
     return launch_bwd_block_fp32(s, q, d_o, lse, delta, k, v, kv_valid_len, sm_scale, dq_acc, dk_acc, dv_acc,

@@ -510,7 +510,8 @@ FwdPlan plan_fwd(const lvx_shape& s) {
   FwdPlan p;
   const int g = s.Hq / s.Hkv;
   p.rows = g * s.Sq;
-  p.m_blocks = (p.rows + 255) / 256;
+  const bool fp32 = s.dtype == LVX_FP32;      // general_tf32.cu: 128 rows a CTA, and 26,000 cycles a tile
+  p.m_blocks = fp32 ? (p.rows + 127) / 128 : (p.rows + 255) / 256;
   p.kv_tiles = (s.Skv + 127) / 128;
   const int qb = q_blocks_of(s);
   const long base = long(p.m_blocks) * s.B * s.Hkv * qb;
@@ -526,7 +527,7 @@ FwdPlan plan_fwd(const lvx_shape& s) {
     const long waves = (ctas + sms - 1) / sms;
     const int tps = (p.kv_tiles + ns - 1) / ns;
     // 3 tiles' worth of fixed cost per CTA (prologue, pipeline fill, epilogue + partial write-out)
-    const double cost = double(waves) * (tps + 3);
+    const double cost = double(waves) * (tps + (fp32 ? 0.5 : 3.0));
     if (cost < best_cost * 0.995) {
       best_cost = cost;
       best = ns;
@@ -545,7 +546,7 @@ int launch_fwd_block(const lvx_shape& s, const FwdPlan& pl, const void* q, const
                      const int32_t* kv_valid_len, float sm_scale, float* o_part, float* ml_part, int* status,
                      cudaStream_t st, const lvx_block_wait* bw, const lvx_bias* bias) {
   if (!(sm_scale > 0.f)) return fail(LVX_ERR_SHAPE, "lvx_fwd_block: sm_scale must be positive");
-  if (s.dtype == LVX_FP32 && bias) return launch_fwd_block_simt(s, pl, q, k, v, kv_valid_len, bias, sm_scale, o_part, ml_part, st);
+  if (s.dtype == LVX_FP32 && bias) return launch_fwd_block_general(s, pl, q, k, v, kv_valid_len, bias, sm_scale, o_part, ml_part, st);
   if (s.dtype == LVX_FP32) return launch_fwd_block_fp32(s, pl, q, k, v, kv_valid_len, sm_scale, o_part, ml_part, st);
   if (pl.rows <= kFewRows && q_blocks_of(s) == 1 && bw == nullptr && bias == nullptr)
     return launch_fwd_rows(s, pl, q, k, v, kv_valid_len, sm_scale, o_part, ml_part, status, st);

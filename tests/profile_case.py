@@ -20,7 +20,7 @@ def main(argv):
     sq, skv = int(argv[1]), int(argv[2])
     iters = int(argv[3]) if len(argv) > 3 else 1
     B, Hq, Hkv = (int(x) for x in argv[4:7]) if len(argv) > 6 else (1, 32, 8)
-    dt = torch.float32 if "fp32" in argv[7:] else torch.bfloat16      # fp32 runs the general FP32-FMA kernels
+    dt = torch.float32 if "fp32" in argv[7:] else torch.bfloat16      # fp32 runs the general kernels
     dev = torch.device("cuda", 0)
     torch.manual_seed(0)
     q = (torch.randn(B, Hq, sq, 128, device=dev) * 0.5).to(dt)
