@@ -182,6 +182,14 @@ int lvx_kv_project(int dtype, const void* x, const void* wk, const void* wv, con
 int lvx_knorm_bwd(int dtype, const void* k, const void* dk, const float* rstd, const void* norm_w, void* dkpre,
                   float* dw, size_t rows, void* stream);
 
+/* The gradients of the projection's outputs as its weight gradients want them: dk_rows, dv_rows [batch, S, Hkv, 128]
+ * (one row per key) from dk, dv [batch, Hkv, S, 128], with the norm's backward applied to dk on the way as in
+ * lvx_knorm_bwd (norm_w NULL: none; dw accumulates otherwise). The reference leaves this to autograd over its modules
+ * (test_llama3.py:394-419). */
+int lvx_kv_project_grad_rows(int dtype, const void* k, const void* dk, const void* dv, const float* rstd,
+                             const void* norm_w, void* dk_rows, void* dv_rows, float* dw, int batch, int Hkv, int S,
+                             void* stream);
+
 /* Merge of `count` finished partial results of the same query block, each computed against a different
  * K/V shard: o_parts fp32 [count][B*Hq*Sq*D], lse_parts fp32 [count][B*Hq*Sq] -> o_out (shape.dtype) and
  * lse_out, with the same stable log-sum-exp merge as lvx_fwd_combine_merge ((0,-inf) is the neutral

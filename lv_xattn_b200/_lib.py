@@ -20,7 +20,7 @@ _DTYPE = {torch.bfloat16: LVX_BF16, torch.float16: LVX_FP16, torch.float32: LVX_
 SYMBOLS = [
     "lvx_version", "lvx_last_error", "lvx_device_status", "lvx_device_status_peek", "lvx_p2p_set_timeout",
     "lvx_query_workspace", "lvx_fwd_block", "lvx_fwd_block_bias", "lvx_bwd_block_bias",
-    "lvx_kv_project", "lvx_knorm_bwd", "lvx_fwd_block_gathered", "lvx_bwd_block_gathered",
+    "lvx_kv_project", "lvx_knorm_bwd", "lvx_kv_project_grad_rows", "lvx_fwd_block_gathered", "lvx_bwd_block_gathered",
     "lvx_fwd_combine_merge", "lvx_bwd_prep", "lvx_bwd_block", "lvx_add_cast", "lvx_selftest_mma",
     "lvx_attn_forward", "lvx_attn_backward", "lvx_local_valid", "lvx_device_status_host",
     "lvx_fwd_block_static", "lvx_fwd_merge_parts", "lvx_sum_cast",
@@ -100,6 +100,8 @@ def load():
     lib.lvx_fwd_merge_parts.argtypes = [sp, fp, fp, ctypes.c_int, ctypes.c_size_t, ctypes.c_size_t, vp, fp, vp]
     lib.lvx_sum_cast.argtypes = [fp, ctypes.c_int, ctypes.c_size_t, vp, ctypes.c_int, ctypes.c_size_t, vp]
     lib.lvx_fwd_block_static.argtypes = [sp, vp, vp, vp, i32p, ctypes.c_float, vp, fp, vp]
+    lib.lvx_kv_project_grad_rows.argtypes = [ctypes.c_int, vp, vp, vp, fp, vp, vp, vp, fp, ctypes.c_int, ctypes.c_int,
+                                             ctypes.c_int, vp]
     lib.lvx_attn_forward.argtypes = [sp, vp, vp, vp, i32p, bp, ctypes.c_float, vp, ctypes.c_size_t, vp, fp, vp]
     lib.lvx_attn_backward.argtypes = [sp, vp, vp, vp, vp, vp, fp, i32p, bp, ctypes.c_float, vp, ctypes.c_size_t, vp, vp, vp, vp]
     lib.lvx_local_valid.argtypes = [vp, ctypes.c_int, ctypes.c_int64, ctypes.c_int, i32p, vp]

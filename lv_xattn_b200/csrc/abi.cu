@@ -457,6 +457,27 @@ int lvx_knorm_bwd(int dtype, const void* k, const void* dk, const float* rstd, c
   return launch_knorm_bwd(dtype, k, dk, rstd, norm_w, dkpre, dw, long(rows), static_cast<cudaStream_t>(stream));
 }
 
+int lvx_kv_project_grad_rows(int dtype, const void* k, const void* dk, const void* dv, const float* rstd,
+                             const void* norm_w, void* dk_rows, void* dv_rows, float* dw, int batch, int Hkv, int S,
+                             void* stream) {
+  const char* who = "lvx_kv_project_grad_rows";
+  if (dtype != LVX_BF16 && dtype != LVX_FP16) return fail(LVX_ERR_DTYPE, "%s: dtype %d unsupported", who, dtype);
+  if (batch < 0 || Hkv <= 0 || S < 0) return fail(LVX_ERR_SHAPE, "%s: negative dimension", who);
+  if (batch == 0 || S == 0) return LVX_OK;
+  LVX_REQUIRE_PTR(k, who);
+  LVX_REQUIRE_PTR(dk, who);
+  LVX_REQUIRE_PTR(dv, who);
+  LVX_REQUIRE_PTR(rstd, who);
+  LVX_REQUIRE_PTR(dk_rows, who);
+  LVX_REQUIRE_PTR(dv_rows, who);
+  if (norm_w) {
+    LVX_REQUIRE_PTR(dw, who);
+    if (reinterpret_cast<uintptr_t>(norm_w) & 7u) return fail(LVX_ERR_ALIGN, "%s: norm_w is not 8-byte aligned", who);
+  }
+  return launch_kvproj_grad_rows(dtype, k, dk, dv, rstd, norm_w, dk_rows, dv_rows, dw, batch, Hkv, S,
+                                 static_cast<cudaStream_t>(stream));
+}
+
 int lvx_fwd_merge_parts(const lvx_shape* s, const float* o_parts, const float* lse_parts, int count,
                         size_t part_stride_o, size_t part_stride_lse, void* o_out, float* lse_out, void* stream) {
   const char* who = "lvx_fwd_merge_parts";

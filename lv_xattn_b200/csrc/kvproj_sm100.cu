@@ -310,14 +310,17 @@ int launch_kv_project(int dtype, const void* x, const void* wk, const void* wv, 
 // every half-warp has four rows in flight and walks on through the tensor with its share of dw in registers, so that a
 // block adds to dw once: with one block per eight rows and an atomic per column and block, the 128 addresses of dw were
 // what the kernel waited for. Measured on 8 heads x 51,232 keys (315 MB): 235 -> 68 us.
+// ROWS: the outputs are laid out [B, S, Hkv, 128], one row of Hkv * 128 columns per key, and dv is brought into the same
+// layout on the way: the weight gradients are then plain [Hkv*128, B*S] x [B*S, hidden] products, which the library runs in
+// 282 us a piece at 51,232 keys against 387 on the transposed head-major gradients (and a copy it makes of those).
 constexpr int KN_ROWS = 4;              // rows in flight per half-warp
 constexpr int KN_BLOCK_ROWS = 16 * KN_ROWS;
 
-template <bool IS_BF16>
+template <bool IS_BF16, bool ROWS>
 __global__ void __launch_bounds__(256)
 knorm_bwd_kernel(const void* __restrict__ k, const void* __restrict__ dk, const float* __restrict__ rstd,
                  const void* __restrict__ norm_w, void* __restrict__ dkpre, float* __restrict__ dw, long rows,
-                 const int* status) {
+                 const void* __restrict__ dv, void* __restrict__ dv_rows, int hkv, int s_len, const int* status) {
   if (status && *reinterpret_cast<const volatile int*>(status) != 0) return;
   __shared__ float s_dw[16][128];
   const int half = threadIdx.x >> 4, l16 = threadIdx.x & 15;      // half-warp of the block, lane in it: columns 8*l16..
@@ -333,14 +336,14 @@ knorm_bwd_kernel(const void* __restrict__ k, const void* __restrict__ dk, const 
   float wf[8], dwl[8];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {      // norm_w is 8-byte aligned
-    const float2 t = unpack16x2<IS_BF16>(reinterpret_cast<const uint32_t*>(norm_w)[l16 * 4 + i]);
+    const float2 t = norm_w ? unpack16x2<IS_BF16>(reinterpret_cast<const uint32_t*>(norm_w)[l16 * 4 + i]) : make_float2(1.f, 1.f);
     wf[2 * i] = t.x;
     wf[2 * i + 1] = t.y;
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) dwl[i] = 0.f;
   for (long base = long(blockIdx.x) * KN_BLOCK_ROWS; base < rows; base += long(gridDim.x) * KN_BLOCK_ROWS) {
-    uint4 kk[KN_ROWS], gg[KN_ROWS];
+    uint4 kk[KN_ROWS], gg[KN_ROWS], vv[ROWS ? KN_ROWS : 1];
     float rs[KN_ROWS];
 #pragma unroll
     for (int u = 0; u < KN_ROWS; ++u) {
@@ -348,6 +351,7 @@ knorm_bwd_kernel(const void* __restrict__ k, const void* __restrict__ dk, const 
       kk[u] = reinterpret_cast<const uint4*>(k)[row * 16 + l16];
       gg[u] = reinterpret_cast<const uint4*>(dk)[row * 16 + l16];
       rs[u] = rstd[row];
+      if constexpr (ROWS) vv[u] = reinterpret_cast<const uint4*>(dv)[row * 16 + l16];
     }
 #pragma unroll
     for (int u = 0; u < KN_ROWS; ++u) {
@@ -361,6 +365,16 @@ knorm_bwd_kernel(const void* __restrict__ k, const void* __restrict__ dk, const 
 #pragma unroll
       for (int off = 8; off > 0; off >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off);
       if (row >= rows) continue;
+      long out = row;
+      if constexpr (ROWS) {
+        const long slab = row / s_len, b = slab / hkv;               // (batch, head)
+        out = (b * s_len + (row - slab * s_len)) * hkv + (slab - b * hkv);
+        reinterpret_cast<uint4*>(dv_rows)[out * 16 + l16] = vv[u];
+        if (norm_w == nullptr) {                                     // no norm: K = Kpre
+          reinterpret_cast<uint4*>(dkpre)[out * 16 + l16] = gg[u];
+          continue;
+        }
+      }
       const float mean = dot * (1.f / 128.f), r = rs[u];
       float o[8];
 #pragma unroll
@@ -369,7 +383,7 @@ knorm_bwd_kernel(const void* __restrict__ k, const void* __restrict__ dk, const 
         o[i] = r * (wf[i] * gf[i] - xhat * mean);
         dwl[i] = fmaf(gf[i], xhat, dwl[i]);
       }
-      reinterpret_cast<uint4*>(dkpre)[row * 16 + l16] =
+      reinterpret_cast<uint4*>(dkpre)[out * 16 + l16] =
           make_uint4(kp_pack<IS_BF16>(o[0], o[1]), kp_pack<IS_BF16>(o[2], o[3]), kp_pack<IS_BF16>(o[4], o[5]),
                      kp_pack<IS_BF16>(o[6], o[7]));
     }
@@ -381,7 +395,7 @@ knorm_bwd_kernel(const void* __restrict__ k, const void* __restrict__ dk, const 
     float a = 0.f;
 #pragma unroll
     for (int w = 0; w < 16; ++w) a += s_dw[w][threadIdx.x];
-    atomicAdd(dw + threadIdx.x, a);
+    if (norm_w) atomicAdd(dw + threadIdx.x, a);
   }
 }
 
@@ -390,10 +404,25 @@ int launch_knorm_bwd(int dtype, const void* k, const void* dk, const float* rstd
   const long blocks = std::min<long>((rows + KN_BLOCK_ROWS - 1) / KN_BLOCK_ROWS, 148 * 6);
   if (blocks == 0) return LVX_OK;
   const int* sp = device_status_ptr();
-  if (dtype == LVX_BF16) knorm_bwd_kernel<true><<<blocks, 256, 0, st>>>(k, dk, rstd, norm_w, dkpre, dw, rows, sp);
-  else knorm_bwd_kernel<false><<<blocks, 256, 0, st>>>(k, dk, rstd, norm_w, dkpre, dw, rows, sp);
+  if (dtype == LVX_BF16) knorm_bwd_kernel<true, false><<<blocks, 256, 0, st>>>(k, dk, rstd, norm_w, dkpre, dw, rows, nullptr, nullptr, 0, 0, sp);
+  else knorm_bwd_kernel<false, false><<<blocks, 256, 0, st>>>(k, dk, rstd, norm_w, dkpre, dw, rows, nullptr, nullptr, 0, 0, sp);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "knorm_bwd launch");
+  return LVX_OK;
+}
+
+int launch_kvproj_grad_rows(int dtype, const void* k, const void* dk, const void* dv, const float* rstd, const void* norm_w,
+                            void* dk_rows, void* dv_rows, float* dw, int batch, int hkv, int s, cudaStream_t st) {
+  const long rows = long(batch) * hkv * s;
+  const long blocks = std::min<long>((rows + KN_BLOCK_ROWS - 1) / KN_BLOCK_ROWS, 148 * 6);
+  if (blocks == 0) return LVX_OK;
+  const int* sp = device_status_ptr();
+  if (dtype == LVX_BF16)
+    knorm_bwd_kernel<true, true><<<blocks, 256, 0, st>>>(k, dk, rstd, norm_w, dk_rows, dw, rows, dv, dv_rows, hkv, s, sp);
+  else
+    knorm_bwd_kernel<false, true><<<blocks, 256, 0, st>>>(k, dk, rstd, norm_w, dk_rows, dw, rows, dv, dv_rows, hkv, s, sp);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "kvproj_grad_rows launch");
   return LVX_OK;
 }
 

@@ -99,6 +99,8 @@ int launch_kv_project(int dtype, const void* x, const void* wk, const void* wv, 
                       cudaStream_t st);
 int launch_knorm_bwd(int dtype, const void* k, const void* dk, const float* rstd, const void* norm_w, void* dkpre,
                      float* dw, long rows, cudaStream_t st);
+int launch_kvproj_grad_rows(int dtype, const void* k, const void* dk, const void* dv, const float* rstd, const void* norm_w,
+                            void* dk_rows, void* dv_rows, float* dw, int batch, int hkv, int s, cudaStream_t st);
 int launch_fwd_merge_parts(const lvx_shape& s, const float* o_parts, const float* lse_parts, int count,
                            size_t stride_o, size_t stride_lse, void* o_out, float* lse_out, cudaStream_t st);
 int launch_sum_cast(const float* parts, int count, size_t stride, void* out, int out_dtype, size_t n, cudaStream_t st);

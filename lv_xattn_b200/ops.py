@@ -372,6 +372,27 @@ def knorm_bwd(k, dk, rstd, norm_weight):
     return dkpre, dw
 
 
+def kv_grad_rows(k, dk, dv, rstd, norm_weight):
+    """The gradients of K and V as the projection's weight gradients want them: (dk_rows, dv_rows [B, S, Hkv*128], dw fp32
+    [128] or None), with the backward of the K norm applied to dk."""
+    _require_cuda(k, dk, dv, rstd, norm_weight)
+    lib = _lib.load()
+    k, dk, dv, rstd = _contig(k), _contig(dk), _contig(dv), _contig(rstd)
+    if dk.dtype != k.dtype or dv.dtype != k.dtype or dk.shape != k.shape or dv.shape != k.shape \
+            or rstd.dtype != torch.float32 or rstd.numel() * 128 != k.numel():
+        raise ValueError("kv_grad_rows: k, dk, dv [B, Hkv, S, 128] in one 16-bit dtype and fp32 rstd with one entry per row")
+    B, H, S, _ = k.shape
+    w = _contig(norm_weight.to(k.dtype)) if norm_weight is not None else None
+    rows = torch.empty(2, B, S, H * 128, dtype=k.dtype, device=k.device)
+    dw = torch.zeros(128, dtype=torch.float32, device=k.device) if w is not None else None
+    _lib.check(lib.lvx_kv_project_grad_rows(_lib.dtype_code(k.dtype), k.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                                            rstd.data_ptr(), None if w is None else w.data_ptr(), rows[0].data_ptr(),
+                                            rows[1].data_ptr(), None if dw is None else dw.data_ptr(), B, H, S,
+                                            _lib.stream_int()), "lvx_kv_project_grad_rows")
+    _count()
+    return rows[0], rows[1], dw
+
+
 def fwd_merge_parts(o_parts, lse_parts, out_dtype, o_out=None, lse_out=None):
     """Merge of finished partials of the same query block: o_parts fp32 [n, B, Hq, Sq, D], lse_parts fp32
     [n, B*Hq, Sq] -> (o [B, Hq, Sq, D] in out_dtype, lse [B*Hq, Sq])."""

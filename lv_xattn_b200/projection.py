@@ -5,9 +5,10 @@ and transposes both to [B, H, S, D], expands them to the query head count and ap
 modules, in forward and again in the backward recompute. At the Llama-3.2-Vision shapes these GEMMs cost about as much
 as the attention itself. `KVProjectFunc` is the same computation as ONE tensor-core GEMM with the per-head RMSNorm
 fused into its epilogue and the result written directly in the [B, Hkv, S, 128] layout the attention kernels read
-(`lvx_kv_project`). Its backward keeps the weight gradients on library GEMMs (torch.matmul): the norm's backward is
-one small kernel of this library (`lvx_knorm_bwd`), then dWk = dKpre^T X and dWv = dV^T X per head, reading dK/dV in
-place (no transposed copies). The states get a gradient only if they ask for one.
+(`lvx_kv_project`). Its backward keeps the weight gradients on library GEMMs (torch.mm): one small kernel of this
+library (`lvx_kv_project_grad_rows`) takes dK and dV from the attention's head-major layout to one row per key, with the
+norm's backward on the way, and dWk = dK^T X and dWv = dV^T X are then one plain product each over all keys of the batch.
+The states get a gradient only if they ask for one.
 """
 from __future__ import annotations
 
@@ -29,22 +30,17 @@ class KVProjectFunc(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dk, dv):
         states, wk, wv, norm_weight, k, rstd = ctx.saved_tensors
-        H = ctx.n_kv_heads
-        B, S, hid = states.shape
-        dk, dv = dk.contiguous(), dv.contiguous()
-        if norm_weight is not None:
-            dkpre, dnw = ops.knorm_bwd(k, dk, rstd, norm_weight)
-        else:
-            dkpre, dnw = dk, None
+        hid = states.shape[-1]
+        dk_rows, dv_rows, dnw = ops.kv_grad_rows(k, dk, dv, rstd, norm_weight)
+        dk_rows, dv_rows = dk_rows.flatten(0, 1), dv_rows.flatten(0, 1)          # [B*S, Hkv*128]
         g_wk = g_wv = g_states = g_nw = None
+        x = states.reshape(-1, hid)
         if ctx.needs_input_grad[1]:
-            # dWk[h] = sum_b dKpre[b,h]^T X[b]: [128, S] x [S, hidden]; the transposed operand is read in place
-            g_wk = sum(torch.matmul(dkpre[b].transpose(-1, -2), states[b]) for b in range(B)).reshape(H * 128, hid)
+            g_wk = torch.mm(dk_rows.t(), x)
         if ctx.needs_input_grad[2]:
-            g_wv = sum(torch.matmul(dv[b].transpose(-1, -2), states[b]) for b in range(B)).reshape(H * 128, hid)
+            g_wv = torch.mm(dv_rows.t(), x)
         if ctx.needs_input_grad[0]:
-            wk3, wv3 = wk.view(H, 128, hid), wv.view(H, 128, hid)
-            g_states = (torch.matmul(dkpre, wk3).sum(1) + torch.matmul(dv, wv3).sum(1))
+            g_states = (torch.mm(dk_rows, wk) + torch.mm(dv_rows, wv)).view(states.shape)
         if norm_weight is not None and ctx.needs_input_grad[3]:
             g_nw = dnw.to(norm_weight.dtype)
         return g_states, g_wk, g_wv, g_nw, None, None
