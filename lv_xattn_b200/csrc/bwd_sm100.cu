@@ -47,7 +47,8 @@
 // two (dO of tile j is free after dV(j), so its successor still arrives under the dS^T half). dV, dK and dQ^T take
 // 16 MMAs instead of 8. The transposed frame suits the bias: a warp's lanes are 32 consecutive keys, so a column's bias
 // values are one 128-byte read. fp16 stays with the general kernel: dS has no bound there, and half of it could
-// fall among fp16's subnormals. Measured at 32 heads, 512 x 6,404: 436 us, 5,177 on the FP32-FMA kernel.
+// fall among fp16's subnormals. Measured at 32 heads, 512 x 6,404: 330 us (436 with half of the bias requested late,
+// at 72 registers; 5,177 on the FP32-FMA kernel that this form replaced).
 #include "lvx_internal.h"
 #include "sm100_prims.cuh"
 #include "block_wait.cuh"
@@ -72,10 +73,10 @@ constexpr int BWD_OFF_STAT = BWD_OFF_DS + BWD_TILE;              // [2][lse2 128
 constexpr int BWD_OFF_BAR = BWD_OFF_STAT + 2 * 256 * 4;
 constexpr int BWD_SMEM = BWD_OFF_BAR + 256;
 constexpr int BWD_COMPUTE_WARPS = 16;
-constexpr int BWD_DRAIN_WARPS = 8;
-constexpr int BWD_WARP_TMA = BWD_COMPUTE_WARPS + BWD_DRAIN_WARPS;
-constexpr int BWD_WARP_MMA = BWD_WARP_TMA + 1;
-constexpr int BWD_THREADS = (BWD_WARP_MMA + 1) * 32;
+// BIAS: four drain warps (dQ^T in two halves each), so that a thread has 88 registers and the bias of a whole tile can be
+// on its way while S^T is
+constexpr int bwd_drain_warps(bool bias) { return bias ? 4 : 8; }
+constexpr int bwd_threads(bool bias) { return (BWD_COMPUTE_WARPS + bwd_drain_warps(bias) + 2) * 32; }
 static_assert(BWD_SMEM <= 232448, "shared memory budget");
 
 constexpr uint32_t TM_DK = 0, TM_DV = 128, TM_X = 256, TM_Y = 384;
@@ -138,9 +139,12 @@ __device__ long long g_bwd_ts[2 * 8 * 16];
 #define BWD_CODE(role, bar) (LVX_DEV_TIMEOUT_BASE | 0x200 | ((role) << 5) | (bar))
 
 template <bool IS_BF16, bool BIAS>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
+__global__ void __launch_bounds__(bwd_threads(BIAS), 1)
 bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
            const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const BwdParams p) {
+  constexpr int BWD_DRAIN_WARPS = bwd_drain_warps(BIAS);
+  constexpr int BWD_WARP_TMA = BWD_COMPUTE_WARPS + BWD_DRAIN_WARPS;
+  constexpr int BWD_WARP_MMA = BWD_WARP_TMA + 1;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + BWD_OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + BB_COUNT);
@@ -268,32 +272,28 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           float stat_after = 0.f;
           if (j + 2 < ntot) stat_after = fetch_stat(j + 2);
           if (warp == 0) BWD_TS(0, 0);
-          // The bias of this key (lane) for the warp's 32 query rows: rows run through the heads of the group, so the
-          // address moves by s_q inside a head and by what is left of s_h at its end. Half of the values are requested
-          // before S^T is waited for, the others while the first half is used.
-          const float* bptr = nullptr;
-          int b_left = 0, b_rows = 0;
-          auto bias16 = [&](float (&b)[16]) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              b[i] = 0.f;
-              if (b_rows > 0 && row_valid) b[i] = __ldg(bptr);
-              --b_rows;
-              bptr += p.bias.s_q;
-              if (--b_left == 0) {
-                b_left = p.bias.sq;
-                bptr += p.bias.s_h - p.bias.sq * p.bias.s_q;
-              }
-            }
-          };
-          float bv[BIAS ? 16 : 1];
+          // The bias of this key (lane) for the warp's 32 query rows, requested before S^T is waited for. Rows run through
+          // the heads of the group: the address moves by s_q inside a head, and past its end on to the next one.
+          float bv[BIAS ? 32 : 1];
           if constexpr (BIAS) {
             const int row = tile_row0(j) + cg * 32, head = row / p.bias.sq, i0 = row - head * p.bias.sq;
-            bptr = p.bias.base + ((p.bw.first_blk + j / nq) % p.nblk) * p.bias.s_blk + (I.slab / p.hkv) * p.bias.s_b +
-                   ((I.slab % p.hkv) * p.bias.g + head) * p.bias.s_h + i0 * p.bias.s_q + (I.kv0 + r) * p.bias.s_kv;
-            b_left = p.bias.sq - i0;
-            b_rows = p.rows - row;
-            bias16(bv);
+            const float* bptr = p.bias.base + ((p.bw.first_blk + j / nq) % p.nblk) * p.bias.s_blk + (I.slab / p.hkv) * p.bias.s_b +
+                                ((I.slab % p.hkv) * p.bias.g + head) * p.bias.s_h + i0 * p.bias.s_q + (I.kv0 + r) * p.bias.s_kv;
+            if (i0 + 32 <= p.bias.sq) {           // one head (then all of the rows exist)
+#pragma unroll
+              for (int i = 0; i < 32; ++i) bv[i] = row_valid ? __ldg(bptr + i * p.bias.s_q) : 0.f;
+            } else {
+              int left = p.bias.sq - i0;
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                bv[i] = row_valid && row + i < p.rows ? __ldg(bptr) : 0.f;
+                bptr += p.bias.s_q;
+                if (--left == 0) {
+                  left = p.bias.sq;
+                  bptr += p.bias.s_h - p.bias.sq * p.bias.s_q;
+                }
+              }
+            }
           }
           // ---------------- P^T half: needs S^T only ----------------
           if (!mbar_wait(&bars[BB_S_FULL], jj & 1, abort_flag, p.status, BWD_CODE(0, BB_S_FULL), p.bw.pipe_limit)) {
@@ -319,11 +319,10 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           for (int i = 0; i < 8; ++i) {
             const float4 l2 = sl[i];
             if constexpr (BIAS) {
-              if (i == 4) bias16(bv);
               float pe[4];
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                const float sc = fmaf(bv[(4 * i + e) & 15], 1.4426950408889634f, __uint_as_float(s[4 * i + e]) * c);
+                const float sc = fmaf(bv[(4 * i + e) & (BIAS ? 31 : 0)], 1.4426950408889634f, __uint_as_float(s[4 * i + e]) * c);
                 pe[e] = row_valid ? ex2f(sc - (e == 0 ? l2.x : e == 1 ? l2.y : e == 2 ? l2.z : l2.w)) : 0.f;
               }
 #pragma unroll
@@ -464,9 +463,10 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     } else if (warp < BWD_WARP_TMA) {
       // =========================== dQ drain warps ===========================
       const int quarter = warp & 3;
-      const int ch = (warp - BWD_COMPUTE_WARPS) >> 2;      // which 64 query columns
+      constexpr int HALVES = 8 / BWD_DRAIN_WARPS;           // halves of the 128 query columns that a warp takes
+      const int ch0 = (warp - BWD_COMPUTE_WARPS) >> 2;      // which 64 query columns (the first of them)
       const int d = quarter * 32 + lane;                    // head-dim index = TMEM lane of dQ^T
-      const uint32_t tY = tmem_base + TM_Y + (static_cast<uint32_t>(quarter * 32) << 16) + ch * 64;
+      const uint32_t tY = tmem_base + TM_Y + (static_cast<uint32_t>(quarter * 32) << 16);
       bool alive = true;
       int jj0 = 0;
       for (int w = blockIdx.x; alive && w < p.nitems; w += gridDim.x) {
@@ -480,15 +480,19 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           }
           tc_fence_after();
           if (warp == BWD_COMPUTE_WARPS) BWD_TS(0, 5);
-          uint32_t v[2][32];
-          tmem_ld32(tY, v[0]);
-          tmem_ld32(tY + 32, v[1]);
-          tc_wait_ld();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars[BB_DQ_FREE]);     // Y is free for the next tile's dP^T
-          if (warp == BWD_COMPUTE_WARPS) BWD_TS(0, 6);
-          {
+#pragma unroll
+          for (int half = 0; half < HALVES; ++half) {
+            const int ch = ch0 + half;
+            uint32_t v[2][32];
+            tmem_ld32(tY + ch * 64, v[0]);
+            tmem_ld32(tY + ch * 64 + 32, v[1]);
+            tc_wait_ld();
+            if (half == HALVES - 1) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bars[BB_DQ_FREE]);     // Y is free for the next tile's dP^T
+            }
+            if (warp == BWD_COMPUTE_WARPS) BWD_TS(0, 6);
             const int row0 = (j % nq) * 128 + ch * 64;
             const int ncols = min(64, p.rows - row0);
             float* dst = p.dq_acc + (size_t(I.slab + ((p.bw.first_blk + j / nq) % p.nblk) * p.kv_slabs) * p.rows + row0) * 128 + d;
@@ -788,9 +792,10 @@ int launch_bwd_block(const lvx_shape& s, const void* q, const void* d_o, const f
   p.nitems = p.kv_tiles * p.kv_slabs;
   dim3 grid(std::min(p.nitems, bwd_num_sms()), 1, 1);      // persistent: one CTA per SM
   cudaError_t e = cudaSuccess;
+  const int threads = bwd_threads(bias != nullptr);
   auto go = [&](auto kern) {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM);
-    if (e == cudaSuccess) kern<<<grid, BWD_THREADS, BWD_SMEM, st>>>(tmQ, tmDO, tmK, tmV, p);
+    if (e == cudaSuccess) kern<<<grid, threads, BWD_SMEM, st>>>(tmQ, tmDO, tmK, tmV, p);
   };
   if (bias) go(bwd_kernel<true, true>);
   else if (s.dtype == LVX_BF16) go(bwd_kernel<true, false>);

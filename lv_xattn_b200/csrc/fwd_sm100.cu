@@ -33,6 +33,11 @@ constexpr int FWD_OFF_K = 2 * FWD_TILE_BYTES;
 constexpr int FWD_OFF_V = FWD_OFF_K + FWD_NS * FWD_TILE_BYTES;
 constexpr int FWD_OFF_BAR = FWD_OFF_V + FWD_NS * FWD_TILE_BYTES;
 constexpr int FWD_SMEM = FWD_OFF_BAR + 256 + 1024;   // + barriers + alignment slack
+// BIAS kernels: one stage for V, and per softmax warp two 32-row x 32-key pieces of the bias (4 KB each)
+constexpr int FWD_OFF_BIAS = FWD_OFF_V + FWD_TILE_BYTES;
+constexpr int FWD_OFF_BAR_B = FWD_OFF_BIAS + 8 * 2 * 4096;
+constexpr int FWD_SMEM_B = FWD_OFF_BAR_B + 256 + 1024;
+static_assert(FWD_SMEM_B <= 232448, "shared memory budget");
 constexpr int FWD_THREADS = 320;
 
 enum {
@@ -83,15 +88,20 @@ __device__ long long g_fwd_ts[3 * 8 * 8];
 // BIAS: a dense additive fp32 bias on the scores (S = scale * q.k + bias). P is then handed to the tensor core as the sum
 // of two 16-bit numbers (the second P V product costs 8 more MMAs per tile), which keeps 16 (bf16) or 22 (fp16) bits of
 // it: the probabilities of this path were fp32 before it used the tensor core, and one 16-bit rounding would show. Every
-// tile takes the exact path, since scores that jump to -inf are what a bias is for. Measured at 32 heads, 512 x 6,404,
-// bf16: 202 us, 2,154 on the FP32-FMA kernel that this form replaces.
+// tile takes the exact path, since scores that jump to -inf are what a bias is for. A thread needs 128 consecutive values
+// of its own row, which read directly would touch 32 lines a load; each warp therefore copies 32 rows x 32 keys at a time,
+// a row's 128 bytes by eight lanes, into a swizzled buffer of its own, two pieces ahead of the one it adds (rows that
+// are not 16-byte aligned, and the ragged last tile, are read directly). V keeps one stage then: its successor has the
+// whole softmax to arrive in. Measured at 32 heads, 512 x 6,404, bf16: 158 us (202 with direct reads, 2,154 on the
+// FP32-FMA kernel that this form replaced).
 template <bool IS_BF16, bool BIAS>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
            const __grid_constant__ CUtensorMap tmV, const FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FWD_OFF_BAR);
+  constexpr int NSV = BIAS ? 1 : FWD_NS;       // V stages
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (BIAS ? FWD_OFF_BAR_B : FWD_OFF_BAR));
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + FB_COUNT);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -150,13 +160,32 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
       const uint32_t tS = tmem_base + wg * 128 + lane_sel;
       const uint32_t tO = tmem_base + 256 + wg * 128 + lane_sel;
       const float c = p.scale_log2;
-      const float c_exp = BIAS ? 1.f : c;          // with a bias the scores are scaled where it is added
       const float* brow = nullptr;                 // this row's bias, from key 0
       if (BIAS) {
         const int prow = mb * 256 + wg * 128 + row_in_tile;
         if (prow < p.rows)
           brow = p.bias.base + blk * p.bias.s_blk + batch * p.bias.s_b +
                  ((kvs % p.hkv) * p.bias.g + prow / p.bias.sq) * p.bias.s_h + (prow % p.bias.sq) * p.bias.s_q;
+      }
+      // Copies keys [col, col + 32) of the warp's 32 bias rows into piece `buf` (rows that do not exist as zeros).
+      auto bias_copy = [&](int col, int buf) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = i * 4 + (lane >> 3), ch = lane & 7;
+          const float* src = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(brow), r));
+          const uint32_t dst = smem_u32(smem + FWD_OFF_BIAS + (warp * 2 + buf) * 4096 + r * 128 + ((ch ^ (r & 7)) << 4));
+          const int bytes = src != nullptr ? 16 : 0;
+          src = src != nullptr ? src + col + ch * 4 : p.bias.base;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+        }
+      };
+      auto bias_staged = [&](int j) { return p.bias_vec && j < n && (tile0 + j + 1) * 128 <= valid; };
+      auto bias_commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+      if (BIAS && bias_staged(0)) {
+        bias_copy(tile0 * 128, 0);
+        bias_commit();
+        bias_copy(tile0 * 128 + 32, 1);
+        bias_commit();
       }
       float m = -INFINITY, l = 0.f;
       bool alive = true;
@@ -174,7 +203,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         // row-max pass at all. Otherwise S is still intact in TMEM and the exact path below runs.
         // A lone warp per scheduler pays the issue time of every instruction in full (measured: 8 cycles per
         // ex2, 4 per cvt.bf16x2, 2 per packed fma/add), so the loop body is kept to the bare minimum.
-        bool done = false;
+        bool done = BIAS;
         if (!BIAS && j > 0 && !(j == n - 1 && last_cols < 128)) {
           uint32_t pk[2][32];
           uint64_t sum_a = f32x2(0.f, 0.f), sum_b = f32x2(0.f, 0.f);
@@ -220,7 +249,105 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             done = true;
           }
         }
-        if (!done) {
+        if constexpr (BIAS) {
+          // 64 scores are held at a time (128 and the pieces of P would not fit the registers): the first 64 get their
+          // bias and go back to TMEM, the others stay; once the maximum is known both become P, the later ones first.
+          constexpr float LOG2E = 1.4426950408889634f;
+          const int col0 = (tile0 + j) * 128;
+          const bool staged = bias_staged(j);
+          uint32_t s[2][32];
+          float mx = -INFINITY;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            tmem_ld32(tS + h * 64, s[0]);
+            tmem_ld32(tS + h * 64 + 32, s[1]);
+            tc_wait_ld();
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int q = 2 * h + e;
+              if (staged) {
+                asm volatile("cp.async.wait_group 1;" ::: "memory");      // all but the piece after this one
+                __syncwarp();
+                const uint8_t* piece = smem + FWD_OFF_BIAS + (warp * 2 + e) * 4096 + lane * 128;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  const float4 b = *reinterpret_cast<const float4*>(piece + ((i ^ (lane & 7)) << 4));
+                  s[e][4 * i] = __float_as_uint(fmaf(b.x, LOG2E, __uint_as_float(s[e][4 * i]) * c));
+                  s[e][4 * i + 1] = __float_as_uint(fmaf(b.y, LOG2E, __uint_as_float(s[e][4 * i + 1]) * c));
+                  s[e][4 * i + 2] = __float_as_uint(fmaf(b.z, LOG2E, __uint_as_float(s[e][4 * i + 2]) * c));
+                  s[e][4 * i + 3] = __float_as_uint(fmaf(b.w, LOG2E, __uint_as_float(s[e][4 * i + 3]) * c));
+                }
+                __syncwarp();
+                if (h == 0) bias_copy(col0 + (q + 2) * 32, e);
+                else if (bias_staged(j + 1)) bias_copy(col0 + 128 + e * 32, e);
+                bias_commit();
+              } else {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                  const int col = col0 + q * 32 + i;
+                  const float b = brow && col < valid ? __ldg(brow + col * p.bias.s_kv) : 0.f;
+                  s[e][i] = col < valid ? __float_as_uint(fmaf(b, LOG2E, __uint_as_float(s[e][i]) * c)) : 0xff800000u;
+                }
+              }
+              float m0 = -INFINITY, m1 = -INFINITY;
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                m0 = fmaxf(m0, __uint_as_float(s[e][i]));
+                m1 = fmaxf(m1, __uint_as_float(s[e][16 + i]));
+              }
+              mx = fmaxf(mx, fmaxf(m0, m1));
+              if (h == 0) tmem_st32(tS + e * 32, s[e]);
+            }
+          }
+          const float m_new = fmaxf(m, mx);
+          const bool grow = m_new > m + 8.f;          // as below
+          float alpha = 1.f;
+          if (grow) {
+            alpha = ex2f(m - m_new);
+            m = m_new;
+            l *= alpha;
+          }
+          if (j > 0 && __any_sync(0xffffffffu, grow)) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              uint32_t o[32];
+              tmem_ld32(tO + q * 32, o);
+              tc_wait_ld();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              tmem_st32(tO + q * 32, o);
+            }
+          }
+          const float moff = (m == -INFINITY) ? 0.f : m;
+          float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+          for (int h = 1; h >= 0; --h) {
+            if (h == 0) {
+              tc_wait_st();
+              tmem_ld32(tS, s[0]);
+              tmem_ld32(tS + 32, s[1]);
+              tc_wait_ld();
+            }
+            // 64 keys: the high halves of P in 32 columns, the low halves in the next 32
+            uint32_t hi[32], lo[32];
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const float a0 = ex2f(__uint_as_float(s[e][2 * i]) - moff), a1 = ex2f(__uint_as_float(s[e][2 * i + 1]) - moff);
+                sum0 += a0;
+                sum1 += a1;
+                const uint32_t w = IS_BF16 ? pack_bf16x2(a0, a1) : pack_f16x2(a0, a1);
+                const float2 t = unpack16x2<IS_BF16>(w);
+                hi[e * 16 + i] = w;
+                lo[e * 16 + i] = IS_BF16 ? pack_bf16x2(a0 - t.x, a1 - t.y) : pack_f16x2(a0 - t.x, a1 - t.y);
+              }
+            tmem_st32(tS + h * 64, hi);
+            tmem_st32(tS + h * 64 + 32, lo);
+          }
+          l += sum0 + sum1;
+        }
+        if (!BIAS && !done) {
           uint32_t s[4][32];
           tmem_ld32(tS + 0, s[0]);
           tmem_ld32(tS + 32, s[1]);
@@ -228,31 +355,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           tmem_ld32(tS + 96, s[3]);
           tc_wait_ld();
           if ((warp & 3) == 0) FWD_TS(wg, 1);
-          if (BIAS) {
-            constexpr float LOG2E = 1.4426950408889634f;
-            const int col0 = (tile0 + j) * 128;
-            if (p.bias_vec && col0 + 128 <= valid) {
-#pragma unroll
-              for (int q = 0; q < 4; ++q)
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                  const float4 b = brow ? __ldg(reinterpret_cast<const float4*>(brow + col0 + q * 32) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-                  s[q][4 * i] = __float_as_uint(fmaf(b.x, LOG2E, __uint_as_float(s[q][4 * i]) * c));
-                  s[q][4 * i + 1] = __float_as_uint(fmaf(b.y, LOG2E, __uint_as_float(s[q][4 * i + 1]) * c));
-                  s[q][4 * i + 2] = __float_as_uint(fmaf(b.z, LOG2E, __uint_as_float(s[q][4 * i + 2]) * c));
-                  s[q][4 * i + 3] = __float_as_uint(fmaf(b.w, LOG2E, __uint_as_float(s[q][4 * i + 3]) * c));
-                }
-            } else {
-#pragma unroll
-              for (int q = 0; q < 4; ++q)
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                  const int col = col0 + q * 32 + i;
-                  const float b = brow && col < valid ? __ldg(brow + col * p.bias.s_kv) : 0.f;
-                  s[q][i] = __float_as_uint(fmaf(b, LOG2E, __uint_as_float(s[q][i]) * c));
-                }
-            }
-          }
           if (j == n - 1 && last_cols < 128) {
 #pragma unroll
             for (int q = 0; q < 4; ++q)
@@ -268,7 +370,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             mx2 = fmaxf(mx2, __uint_as_float(s[2][i]));
             mx3 = fmaxf(mx3, __uint_as_float(s[3][i]));
           }
-          const float m_new = fmaxf(m, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * c_exp);
+          const float m_new = fmaxf(m, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * c);
           // The running max is only raised when it would grow by more than 2^8; P then stays below 256
           // and the accumulator rarely needs rescaling. (m, l, O) remain mutually consistent.
           const bool grow = m_new > m + 8.f;
@@ -294,25 +396,19 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            uint32_t pk[32], lo[BIAS ? 32 : 1];
+            uint32_t pk[32];
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-              const float a0 = ex2f(fmaf(__uint_as_float(s[2 * h][2 * i]), c_exp, -moff));
-              const float a1 = ex2f(fmaf(__uint_as_float(s[2 * h][2 * i + 1]), c_exp, -moff));
-              const float b0 = ex2f(fmaf(__uint_as_float(s[2 * h + 1][2 * i]), c_exp, -moff));
-              const float b1 = ex2f(fmaf(__uint_as_float(s[2 * h + 1][2 * i + 1]), c_exp, -moff));
+              const float a0 = ex2f(fmaf(__uint_as_float(s[2 * h][2 * i]), c, -moff));
+              const float a1 = ex2f(fmaf(__uint_as_float(s[2 * h][2 * i + 1]), c, -moff));
+              const float b0 = ex2f(fmaf(__uint_as_float(s[2 * h + 1][2 * i]), c, -moff));
+              const float b1 = ex2f(fmaf(__uint_as_float(s[2 * h + 1][2 * i + 1]), c, -moff));
               sum0 += a0 + a1;
               sum1 += b0 + b1;
               pk[i] = IS_BF16 ? pack_bf16x2(a0, a1) : pack_f16x2(a0, a1);
               pk[16 + i] = IS_BF16 ? pack_bf16x2(b0, b1) : pack_f16x2(b0, b1);
-              if constexpr (BIAS) {
-                const float2 ha = unpack16x2<IS_BF16>(pk[i]), hb = unpack16x2<IS_BF16>(pk[16 + i]);
-                lo[i] = IS_BF16 ? pack_bf16x2(a0 - ha.x, a1 - ha.y) : pack_f16x2(a0 - ha.x, a1 - ha.y);
-                lo[16 + i] = IS_BF16 ? pack_bf16x2(b0 - hb.x, b1 - hb.y) : pack_f16x2(b0 - hb.x, b1 - hb.y);
-              }
             }
             tmem_st32(tS + h * 32, pk);
-            if constexpr (BIAS) tmem_st32(tS + 64 + h * 32, lo);
           }
           l += sum0 + sum1;
         }
@@ -369,10 +465,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           tma_load_3d(smem + FWD_OFF_K + s * FWD_TILE_BYTES, &tmK, &bars[FB_K_FULL + s], 0, y, kvs);
           tma_load_3d(smem + FWD_OFF_K + s * FWD_TILE_BYTES + FWD_HALF_BYTES, &tmK, &bars[FB_K_FULL + s], 64, y, kvs);
           k_issued = j + 1;
-          if (!mbar_wait(&bars[FB_V_EMPTY + s], ph ^ 1, abort_flag, p.status, FWD_CODE(2, FB_V_EMPTY), p.bw.pipe_limit)) break;
-          mbar_arrive_expect_tx(&bars[FB_V_FULL + s], FWD_TILE_BYTES);
-          tma_load_3d(smem + FWD_OFF_V + s * FWD_TILE_BYTES, &tmV, &bars[FB_V_FULL + s], 0, y, kvs);
-          tma_load_3d(smem + FWD_OFF_V + s * FWD_TILE_BYTES + FWD_HALF_BYTES, &tmV, &bars[FB_V_FULL + s], 64, y, kvs);
+          const int sv = j % NSV;
+          if (!mbar_wait(&bars[FB_V_EMPTY + sv], ((j / NSV) & 1) ^ 1, abort_flag, p.status, FWD_CODE(2, FB_V_EMPTY), p.bw.pipe_limit)) break;
+          mbar_arrive_expect_tx(&bars[FB_V_FULL + sv], FWD_TILE_BYTES);
+          tma_load_3d(smem + FWD_OFF_V + sv * FWD_TILE_BYTES, &tmV, &bars[FB_V_FULL + sv], 0, y, kvs);
+          tma_load_3d(smem + FWD_OFF_V + sv * FWD_TILE_BYTES + FWD_HALF_BYTES, &tmV, &bars[FB_V_FULL + sv], 64, y, kvs);
           v_issued = j + 1;
         }
         // A CTA that is giving up must not leave while a copy into its shared memory is in flight.
@@ -383,7 +480,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           };
           if (q_here) drain(&bars[FB_Q_FULL], 0);
           for (int j = max(0, k_issued - FWD_NS); j < k_issued; ++j) drain(&bars[FB_K_FULL + j % FWD_NS], (j / FWD_NS) & 1);
-          for (int j = max(0, v_issued - FWD_NS); j < v_issued; ++j) drain(&bars[FB_V_FULL + j % FWD_NS], (j / FWD_NS) & 1);
+          for (int j = max(0, v_issued - NSV); j < v_issued; ++j) drain(&bars[FB_V_FULL + j % NSV], (j / NSV) & 1);
         }
       }
     } else {
@@ -417,14 +514,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         auto issue_pv = [&](int i, int stage, bool first) {
           const uint32_t b_lo = umma_desc_lo(sV + stage * FWD_TILE_BYTES, FWD_HALF_BYTES);
           if (elect_one()) {
+            // A: P, 8 columns per k-step; with BIAS 32 columns of high halves and 32 of low halves per 64 keys
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
-              umma_ts_f16(tmem_base + 256 + i * 128, tmem_base + i * 128 + kk * 8,
+              umma_ts_f16(tmem_base + 256 + i * 128, tmem_base + i * 128 + kk * 8 + (BIAS ? (kk >> 2) * 32 : 0),
                           umma_desc_join(b_lo + ((kk * 2048) >> 4), HI), IDESC_PV, (!first) || kk > 0);
-            if constexpr (BIAS) {      // the low half of P
+            if constexpr (BIAS) {
 #pragma unroll
               for (int kk = 0; kk < 8; ++kk)
-                umma_ts_f16(tmem_base + 256 + i * 128, tmem_base + i * 128 + 64 + kk * 8,
+                umma_ts_f16(tmem_base + 256 + i * 128, tmem_base + i * 128 + 32 + kk * 8 + (kk >> 2) * 32,
                             umma_desc_join(b_lo + ((kk * 2048) >> 4), HI), IDESC_PV, true);
             }
           }
@@ -447,8 +545,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           commit(&bars[FB_K_EMPTY + 0]);
         }
         for (int j = 0; ok && j < n; ++j) {
-          const int s = j % FWD_NS;
-          const uint32_t ph = (j / FWD_NS) & 1;
+          const int s = j % NSV;                       // V stage
+          const uint32_t ph = (j / NSV) & 1;
           const int s1 = (j + 1) % FWD_NS;
           const uint32_t ph1 = ((j + 1) / FWD_NS) & 1;
 #pragma unroll
@@ -587,8 +685,9 @@ int launch_fwd_block(const lvx_shape& s, const FwdPlan& pl, const void* q, const
   dim3 grid(pl.m_blocks, qb * s.B * s.Hkv, pl.nsplit);
   cudaError_t e = cudaSuccess;
   auto go = [&](auto kern) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM);
-    if (e == cudaSuccess) kern<<<grid, FWD_THREADS, FWD_SMEM, st>>>(tmQ, tmK, tmV, p);
+    const int smem = bias ? FWD_SMEM_B : FWD_SMEM;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) kern<<<grid, FWD_THREADS, smem, st>>>(tmQ, tmK, tmV, p);
   };
   if (s.dtype == LVX_BF16) bias ? go(fwd_kernel<true, true>) : go(fwd_kernel<true, false>);
   else bias ? go(fwd_kernel<false, true>) : go(fwd_kernel<false, false>);
