@@ -50,13 +50,21 @@ static int* host_status_word(cudaStream_t st) {
   if (g_host_status[dev]) return g_host_status[dev];
   int* sp = status_ptr();
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (!sp || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return nullptr;
+  // what fails here must not show up as the error of a later launch: the host word is a convenience
+  if (!sp || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
   void *h = nullptr, *d = nullptr;
-  if (cudaHostAlloc(&h, 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+  if (cudaHostAlloc(&h, 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
   *static_cast<volatile int*>(h) = 0;
   if (cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess ||
       cudaMemcpy(sp + 2, &d, sizeof(d), cudaMemcpyHostToDevice) != cudaSuccess) {
     cudaFreeHost(h);
+    (void)cudaGetLastError();
     return nullptr;
   }
   g_host_status[dev] = static_cast<int*>(h);
