@@ -2,8 +2,8 @@
 //   fwd_combine_kernel  split-KV partials (+) travelling (O, lse)  ->  (O, lse)
 //   bwd_prep_kernel     delta = rowsum(O * dO)
 //   add_cast_kernel     out = cast(a + b)
-// One warp handles one 128-wide row with float4 / 8-byte accesses, so every access is a full 512-byte
-// (fp32) or 256-byte (16-bit) coalesced row.
+// A row of 128 values is read by one warp (fp32) or half a warp (16 bits), 16 bytes a lane, so that every access is a full
+// coalesced 512- or 256-byte row.
 #include "lvx_internal.h"
 #include "sm100_prims.cuh"
 #include <cuda_bf16.h>
