@@ -273,13 +273,14 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           if (j + 2 < ntot) stat_after = fetch_stat(j + 2);
           if (warp == 0) BWD_TS(0, 0);
           // The bias of this key (lane) for the warp's 32 query rows, requested before S^T is waited for. Rows run through
-          // the heads of the group: the address moves by s_q inside a head, and past its end on to the next one.
+          // the heads of the group: the address moves by s_q inside a head, and past its end on to the next one. The last
+          // tile may be partly filled: past the group's last head there is no row and no bias to read.
           float bv[BIAS ? 32 : 1];
           if constexpr (BIAS) {
             const int row = tile_row0(j) + cg * 32, head = row / p.bias.sq, i0 = row - head * p.bias.sq;
             const float* bptr = p.bias.base + ((p.bw.first_blk + j / nq) % p.nblk) * p.bias.s_blk + (I.slab / p.hkv) * p.bias.s_b +
                                 ((I.slab % p.hkv) * p.bias.g + head) * p.bias.s_h + i0 * p.bias.s_q + (I.kv0 + r) * p.bias.s_kv;
-            if (i0 + 32 <= p.bias.sq) {           // one head (then all of the rows exist)
+            if (head < p.bias.g && i0 + 32 <= p.bias.sq) {      // one head that exists: so do all 32 rows
 #pragma unroll
               for (int i = 0; i < 32; ++i) bv[i] = row_valid ? __ldg(bptr + i * p.bias.s_q) : 0.f;
             } else {

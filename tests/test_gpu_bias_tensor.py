@@ -66,6 +66,31 @@ def test_bias_forms(cuda_device, shape, kind, dtype):
     _parity.assert_grads_16bit((dq, dk, dv), ref[2:], label)
 
 
+@pytest.mark.parametrize("shape", [(2, 4, 2, 77, 388), (1, 2, 2, 300, 200), (1, 1, 1, 64, 130), (1, 3, 1, 96, 129)])
+def test_last_tile_reads_no_bias_of_rows_that_do_not_exist(cuda_device, shape):
+    """The packed rows end inside a 128-row tile. The per-head bias is a leading slice of a larger buffer of NaN, so that a
+    value read past the last head's rows shows in dK and dV (a NaN P times a zero dO)."""
+    from lv_xattn_b200 import ops, _lib
+    B, Hq, Hkv, Sq, Skv = shape
+    q, k, v, do = orc.make_inputs(B, Hq, Hkv, Sq, Skv, 128, 75, torch.bfloat16)
+    n = B * Hq * Sq * Skv
+    buf = torch.full((n + 256 * Skv,), float("nan"))
+    bias = buf[:n].view(B, Hq, Sq, Skv)
+    bias.copy_(torch.randn(B, Hq, Sq, Skv, generator=torch.Generator().manual_seed(76)))
+    ref = orc.attention_fwd_bwd(q, k, v, do, SCALE, None, bias=bias)
+    bias = buf.to(cuda_device)[:n].view(B, Hq, Sq, Skv)
+    qd, kd, vd, dod = (t.to(cuda_device) for t in (q, k, v, do))
+    o, lse = ops.fwd_block(qd, kd, vd, SCALE, bias=bias)
+    delta = ops.bwd_prep(o, dod)
+    dq = torch.zeros(B, Hq, Sq, 128, device=cuda_device)
+    dk, dv = torch.empty_like(kd), torch.empty_like(vd)
+    ops.bwd_block(qd, dod, lse, delta, kd, vd, SCALE, dq, dk, dv, "final", None, bias=bias)
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    _parity.assert_close(o.float().cpu(), ref[0], "o", f"bias_tail{shape}", *_parity.BF16["o"])
+    _parity.assert_grads_16bit((dq, dk, dv), ref[2:], f"bias_tail{shape}")
+
+
 def test_two_part_operands(cuda_device):
     """fp32 outputs against 64 bits. P and dS are held to 2^-17 of each value (two bf16 numbers), the scores to fp32 sums
     over 128 products; 2^-15 leaves a factor of four. One bf16 rounding would show at 2^-9."""
