@@ -71,15 +71,31 @@ fwd_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FR_OFF_BAR);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + FR_COUNT);
+  volatile int* poisoned = abort_flag + 1;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int split = blockIdx.x, slab = blockIdx.y;
+  // The status word may be set by another CTA or stream at any moment: one thread reads it, and the CTA leaves or stays as
+  // a whole. Warps that went on alone would meet barriers that nobody initialised and wait for the others at bar.sync.
+  int word = 0;
+  if (tid == 0) word = *reinterpret_cast<volatile int*>(p.status);
   int valid = p.skv;
   if (p.kv_valid_len) valid = min(valid, max(0, p.kv_valid_len[slab / p.hkv]));
   const int valid_tiles = (valid + 127) >> 7;
   const int tile0 = split * p.tiles_per_split;
   const int n = max(0, min(tile0 + p.tiles_per_split, valid_tiles) - tile0);
-  if (*reinterpret_cast<volatile int*>(p.status) != 0) return;
+  if (tid == 0) {
+    for (int s = 0; s < FR_STAGES; ++s) {
+      mbar_init(&bars[FR_K_FULL + s], 1);
+      mbar_init(&bars[FR_V_FULL + s], 1);
+      mbar_init(&bars[FR_EMPTY + s], FR_WARPS);
+    }
+    *abort_flag = 0;
+    *poisoned = word;
+    fence_mbar_init();
+  }
+  __syncthreads();
+  if (*poisoned != 0) return;
 
   float* o_dst = p.o_part + (size_t(slab) * p.nsplit + split) * p.rows * 128;
   float* ml_dst = p.ml_part + (size_t(slab) * p.nsplit + split) * p.rows * 2;
@@ -88,16 +104,6 @@ fwd_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     for (int i = tid; i < p.rows; i += FR_THREADS) reinterpret_cast<float2*>(ml_dst)[i] = make_float2(-INFINITY, 0.f);
     return;
   }
-  if (tid == 0) {
-    for (int s = 0; s < FR_STAGES; ++s) {
-      mbar_init(&bars[FR_K_FULL + s], 1);
-      mbar_init(&bars[FR_V_FULL + s], 1);
-      mbar_init(&bars[FR_EMPTY + s], FR_WARPS);
-    }
-    *abort_flag = 0;
-    fence_mbar_init();
-  }
-  __syncthreads();
 
   if (warp == FR_WARPS) {
     // =========================== TMA producer ===========================

@@ -41,3 +41,26 @@ def test_key_edges(cuda_device, skv):
 def test_key_padding_and_large_scores(cuda_device, Sq):
     # a sample without any valid key, ranges that end inside a warp's keys; queries scaled so that the running max jumps
     run_and_check(cuda_device, 4, 4, 1, Sq, 900, torch.bfloat16, valid=[900, 0, 387, 5], gain=16.0, label=f"rows_pad{Sq}")
+
+
+@pytest.mark.parametrize("skv", [100, 5000])
+def test_word_already_set(cuda_device, skv):
+    """A wait that ran out earlier (a flag that nothing sets, with the limit at 1 ms) has left its code in the status word:
+    the whole kernel leaves at once and writes nothing, and works again once the word has been cleared."""
+    from lv_xattn_b200 import ops, _lib
+    q, k, v, _ = (t.to(cuda_device) for t in orc.make_inputs(2, 8, 2, 5, skv, 128, 12, torch.bfloat16))
+    o, lse = ops.fwd_block(q, k, v, SCALE)
+    lib = _lib.load()
+    lib.lvx_p2p_set_timeout(0.001)
+    try:
+        ops.p2p_wait(torch.zeros(8 * 16, dtype=torch.int32, device=cuda_device), 1, 0, 1)
+        part = ops.fwd_partials(q, k, v, SCALE)
+        part.ws.fill_(7)
+        ops.fwd_partials(q, k, v, SCALE)
+        torch.cuda.synchronize()
+        assert (part.ws == 7).all()
+    finally:
+        lib.lvx_p2p_set_timeout(120.0)
+        assert _lib.device_status() != 0                 # reading clears it
+    again = ops.fwd_block(q, k, v, SCALE)
+    assert torch.equal(again[0], o) and torch.equal(again[1], lse)
