@@ -77,11 +77,11 @@ int lvx_device_status(void* stream, int* status_out);
  * without synchronising; the reference would simply block for ever (lv_xattn/async_communication.py:301-305). */
 int lvx_device_status_peek(void* stream, int* host_out);
 
-/* The host's own copy of the current device's word: *host_word points to an int that lvx_fwd_combine_merge and
- * lvx_add_cast (the last kernels of a forward and a backward) write when they find the word set (mapped pinned memory, kept
+/* The host's own copy of the current device's word: *host_word points to an int that lvx_fwd_combine_merge, lvx_add_cast
+ * and the fp32 backward block (the last kernels of a pass) write when they find the word set (mapped pinned memory, kept
  * for the life of the process, cleared by lvx_device_status), so that a host loop can look at it before every call at the
- * price of a memory read. Set up by the first call; NULL if that call comes while `stream`
- * is being captured. No reference counterpart (its waits are unbounded, lv_xattn/async_communication.py:301-305). */
+ * price of a memory read. Set up by the first call; NULL if that call comes while `stream` is being captured. No reference
+ * counterpart (its waits are unbounded, lv_xattn/async_communication.py:301-305). */
 int lvx_device_status_host(void* stream, const int** host_word);
 
 /* Global key-padding lengths -> this rank's: out[i] = clamp(valid_len[i] - first_key, 0, skv) for `count` host values,

@@ -21,18 +21,6 @@ __device__ __forceinline__ bool poisoned(const int* status) {
   return status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0;
 }
 
-// The last kernel of a forward or backward pass (combine, add_cast) also tells the host: status[2..3] hold the address of
-// the host's copy of the word where the library has set one up, and a pass that found the word set writes it there. The
-// host then notices with a read of its own memory, and a GPU on which nothing fails does nothing for it.
-__device__ __forceinline__ void publish_status(const int* status) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  int* host = *reinterpret_cast<int* const volatile*>(status + 2);
-  if (host != nullptr) {
-    *reinterpret_cast<volatile int*>(host) = *reinterpret_cast<const volatile int*>(status);
-    __threadfence_system();
-  }
-}
-
 template <int OUT>  // 0 bf16, 1 fp16, 2 fp32
 __device__ __forceinline__ void store4(void* base, size_t idx4, float4 v) {
   if (OUT == 2) {
@@ -139,7 +127,7 @@ fwd_combine_kernel(const float* __restrict__ o_part, const float* __restrict__ m
     }
   }
   if (bad) {
-    publish_status(status);
+    if (lane == 0) publish_status(status);
     return;
   }
   float4 acc = a.v;
@@ -305,7 +293,7 @@ __global__ void __launch_bounds__(256)
 add_cast_kernel(const float* __restrict__ a, const float* __restrict__ b, void* __restrict__ out, size_t n4, size_t n,
                 const int* status) {
   if (poisoned(status)) {
-    publish_status(status);
+    if ((threadIdx.x & 31) == 0) publish_status(status);
     return;
   }
   const size_t stride = size_t(gridDim.x) * blockDim.x;

@@ -304,7 +304,11 @@ template <typename T>
 __global__ void __launch_bounds__(256, 1)
 fp32_bwd_kernel(const Fp32BwdParams p) {
   constexpr bool EX = sizeof(T) == 2;          // 16-bit inputs are exact in tf32
-  if (p.status && *reinterpret_cast<const volatile int*>(p.status) != 0) return;
+  // This kernel ends an fp32 backward (dQ is accumulated where it is wanted), so it also tells the host.
+  if (p.status && __syncthreads_or(*reinterpret_cast<const volatile int*>(p.status) != 0)) {
+    if (threadIdx.x == 0) publish_status(p.status);
+    return;
+  }
   extern __shared__ __align__(16) float sm[];
   float* sK = sm;
   float* sV = sK + GT_TILE;

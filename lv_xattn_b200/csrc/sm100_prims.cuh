@@ -334,6 +334,18 @@ __device__ __forceinline__ float2 unpack16x2(uint32_t v) {
   if (IS_BF16) return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
   return __half22float2(*reinterpret_cast<const __half2*>(&v));
 }
+// The last kernel of a forward or backward pass (combine, add_cast, the general backward where dQ needs no cast) also tells
+// the host: status[2..3] hold the address of the host's copy of the word where the library has set one up, and every warp
+// that found the word set and left its work undone writes it there (the word may be set while the kernel runs, so that no
+// one block can speak for all). The host then notices with a read of its own memory, and a GPU on which nothing fails does
+// nothing for it.
+__device__ __forceinline__ void publish_status(const int* status) {
+  int* host = *reinterpret_cast<int* const volatile*>(status + 2);
+  if (host != nullptr) {
+    *reinterpret_cast<volatile int*>(host) = *reinterpret_cast<const volatile int*>(status);
+    __threadfence_system();
+  }
+}
 // Two fp32 lanes per instruction (sm_100 packed arithmetic): halves the issue slots of the softmax inner loops.
 __device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
   uint64_t r;

@@ -87,3 +87,35 @@ def test_a_wait_that_ran_out_is_noticed_at_the_next_call(cuda_device):
     finally:
         lib.lvx_p2p_set_timeout(120.0)
         _lib.device_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("bias", [False, True])
+def test_a_pass_that_found_the_word_set_is_reported(cuda_device, dtype, bias):
+    """Either pass of every type, each as the first one after the wait: what it left unwritten must not go unnoticed."""
+    import lv_xattn_b200 as lvx
+    from lv_xattn_b200 import ops, _lib, peer_memory as pm
+    from lv_xattn_b200.async_communication import P2PTimeoutError
+    q, k, v, do = (t.to(cuda_device) for t in orc.make_inputs(1, 2, 1, 70, 300, 128, 84, dtype))
+    kw = {}
+    if bias:
+        kw.update(bias_func=lambda t: t, local_bias_args=[torch.randn(1, 1, 70, 300, device=cuda_device)], remote_bias_args=[])
+    good = both_passes(q, k, v, do, **kw)
+    pm.check_device_status()
+    flags = torch.zeros(8 * 16, dtype=torch.int32, device=cuda_device)
+    lib = _lib.load()
+    lib.lvx_p2p_set_timeout(0.001)
+    try:
+        for backward in (True, False):
+            ops.p2p_wait(flags, 1, 0, 1)
+            if backward:
+                lvx._attn_backward(do, q, k, v, good[0], good[1], False, SCALE, None, "flash", **kw)
+            else:
+                lvx._attn_forward(q, k, v, False, SCALE, None, **kw)
+            with pytest.raises(P2PTimeoutError):
+                pm.check_device_status()
+            pm.check_device_status()
+        assert torch.equal(both_passes(q, k, v, do, **kw)[0], good[0])
+    finally:
+        lib.lvx_p2p_set_timeout(120.0)
+        _lib.device_status()
