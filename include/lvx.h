@@ -29,7 +29,9 @@ extern "C" {
 
 #define LVX_ABI_VERSION 1
 
-enum lvx_dtype { LVX_BF16 = 0, LVX_FP16 = 1, LVX_FP32 = 2 /* fp32 accuracy: products in three tf32 parts, fp32 sums */ };
+/* LVX_FP32: fp32 accuracy, products in three tf32 parts, fp32 sums. Infinities, NaN and values up to the largest float
+ * come out where a plain sum has them, except that an infinity times a value of 4,096 or more may give NaN. */
+enum lvx_dtype { LVX_BF16 = 0, LVX_FP16 = 1, LVX_FP32 = 2 };
 
 enum lvx_error {
   LVX_OK = 0,

@@ -64,3 +64,24 @@ def test_word_already_set(cuda_device, skv):
         assert _lib.device_status() != 0                 # reading clears it
     again = ops.fwd_block(q, k, v, SCALE)
     assert torch.equal(again[0], o) and torch.equal(again[1], lse)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_infinities_and_nan(cuda_device, dtype):
+    """Those of V come out in the columns where a plain sum has them, and a key that scores -inf counts as no key."""
+    from lv_xattn_b200 import ops
+    q, k, v, _ = orc.make_inputs(1, 6, 3, 7, 700, 128, 13, dtype)
+    q[..., 0] = q[..., 0].abs() + 0.125
+    k[0, 0, 130, 0] = float("-inf")
+    v[0, 0, 3, 5] = float("inf")
+    v[0, 1, 300, 6] = float("-inf")
+    v[0, 1, 301, 7] = float("nan")
+    k6, v6 = (t.double().repeat_interleave(2, 1) for t in (k, v))
+    o6 = (q.double() @ k6.transpose(-1, -2) * SCALE).softmax(-1) @ v6
+    o, lse = ops.fwd_block(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), SCALE)
+    o = o.double().cpu()
+    for at in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(at(o), at(o6))
+    fin = torch.isfinite(o6)
+    _parity.assert_close(o[fin], o6[fin], "o", f"rows_extremes{dtype}", *_parity.BF16["o"])
+    assert torch.isfinite(lse).all()
