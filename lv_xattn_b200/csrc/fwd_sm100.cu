@@ -86,8 +86,8 @@ __device__ long long g_fwd_ts[3 * 8 * 8];
 #define FWD_CODE(role, bar) (LVX_DEV_TIMEOUT_BASE | 0x100 | ((role) << 5) | (bar))
 
 // BIAS: a dense additive fp32 bias on the scores (S = scale * q.k + bias). P is then handed to the tensor core as the sum
-// of two 16-bit numbers (the second P V product costs 8 more MMAs per tile), which keeps 16 (bf16) or 22 (fp16) bits of
-// it: the probabilities of this path were fp32 before it used the tensor core, and one 16-bit rounding would show. Every
+// of two 16-bit numbers (the second P V product costs 8 more MMAs per tile), which keeps 16 (bf16) or 22 (fp16, but
+// nothing below 2^-36 of the row's maximum) bits of it: the probabilities of this path were fp32 before it used the tensor core, and one 16-bit rounding would show. Every
 // tile takes the exact path, since scores that jump to -inf are what a bias is for. A thread needs 128 consecutive values
 // of its own row, which read directly would touch 32 lines a load; each warp therefore copies 32 rows x 32 keys at a time,
 // a row's 128 bytes by eight lanes, into a swizzled buffer of its own, two pieces ahead of the one it adds (rows that
@@ -299,12 +299,16 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
               if (h == 0) tmem_st32(tS + e * 32, s[e]);
             }
           }
-          const float m_new = fmaxf(m, mx);
-          const bool grow = m_new > m + 8.f;          // as below
+          // The reference is raised when the maximum has outgrown it, as below. In fp16 it is put 2^12 under the maximum, so
+          // that P stays below 2^15 and its two halves reach down to 2^-36 of the maximum: with the maximum itself as the
+          // reference everything below 2^-24 of it would be lost, which is all of a row's output where one key dominates
+          // and its value is small. (bf16 has fp32's range.)
+          constexpr float SLACK = IS_BF16 ? 8.f : 15.f, UNDER = IS_BF16 ? 0.f : 12.f;
+          const bool grow = mx > m + SLACK;
           float alpha = 1.f;
           if (grow) {
-            alpha = ex2f(m - m_new);
-            m = m_new;
+            alpha = ex2f(m - (mx - UNDER));
+            m = mx - UNDER;
             l *= alpha;
           }
           if (j > 0 && __any_sync(0xffffffffu, grow)) {

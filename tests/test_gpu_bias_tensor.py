@@ -112,3 +112,26 @@ def test_two_part_operands(cuda_device):
     for name, got, ref in (("o", o, o6), ("dq", dq, dq6), ("dk", dk, dk6), ("dv", dv, dv6)):
         err = ((got.cpu().double() - ref).norm() / ref.norm()).item()
         assert err <= 2.0 ** -15, (name, err)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("below", [18.3, 25.5])
+@pytest.mark.parametrize("at", [0, 700, 5999])
+def test_small_probabilities_beside_a_dominant_key(cuda_device, dtype, below, at):
+    """One key, whose value is zero, outweighs every other one by 2^18 or 2^25: the output is what the others add up to.
+    In fp16, P relative to the row's maximum would be subnormal or nothing there. P is held to 2^-25 of 2^-12 of the
+    maximum, i.e. to 2^-11.5 of the smaller probabilities here, and the output is rounded to 16 bits."""
+    from lv_xattn_b200 import ops
+    B, H, Sq, Skv = 1, 2, 40, 6000
+    g = torch.Generator().manual_seed(77)
+    q = torch.zeros(B, H, Sq, 128, dtype=dtype)
+    k = torch.empty(B, H, Skv, 128).normal_(0, 0.5, generator=g).to(dtype)
+    v = (1 + torch.empty(B, H, Skv, 128).normal_(0, 0.5, generator=g)).to(dtype)
+    v[:, :, at] = 0
+    bias = torch.full((1, 1, Sq, Skv), -below * math.log(2.0))
+    bias[..., at] = 0
+    ref = bias.double().expand(B, H, Sq, Skv).softmax(-1) @ v.double()
+    o, lse = ops.fwd_block(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), SCALE, bias=bias.to(cuda_device))
+    err = ((o.cpu().double() - ref).norm() / ref.norm()).item()
+    assert err <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10), err
+    assert (lse.cpu().double() - torch.logsumexp(bias.double()[0, 0], -1)).abs().max() <= 1e-5
