@@ -383,8 +383,7 @@ def _attn_backward(do, q, k, v, o, L, causal, sm_scale, comm_mode, backward_engi
         dk = torch.empty(B, Hkv, Skv, D, dtype=dt, device=dev)
         dv = torch.empty(B, Hkv, Skv, D, dtype=dt, device=dev)
         bias = _build_bias(bias_func, local_bias_args, remote_bias_args, qc, kc)
-        scratch = get_slabs("bwd_dq_delta", (n_q + n_r) * 4, dev, 1)[0]
-        ops.attn_backward(doc, qc, kc, vc, oc, Lc, sm_scale, kvl, bias, scratch, dq, dk, dv)
+        ops.attn_backward(doc, qc, kc, vc, oc, Lc, sm_scale, kvl, bias, dq, dk, dv)
         return dq, dk, dv
     delta = ops.bwd_prep(oc, doc)                       # once, at home; travels instead of O
     dq = torch.empty(B, Hq, Sq, D, dtype=dt, device=dev)

@@ -215,20 +215,22 @@ def attn_forward(q, k, v, sm_scale, kv_valid_len, bias, o, lse) -> None:
         if len(_fwd_bytes) >= 4096:
             _fwd_bytes.clear()
         nbytes = _fwd_bytes[key] = _lib.query_workspace(shp)[0]
-    ws = _workspace(q.device, nbytes)
+    # of the caching allocator, which knows streams, threads and graph captures: a buffer kept per device is none of a
+    # call's own where another stream or thread is between its two launches
+    ws = lse.new_empty(nbytes // 4)
     if kv_valid_len is not None and kv_valid_len.numel() != shp.B:
         raise ValueError("kv_valid_len must be an int32 tensor with one entry per batch element")
     bv, keep = _bias_view(bias, q, k) if bias is not None else (None, None)
     _lib.check(lib.lvx_attn_forward(ctypes.byref(shp), q.data_ptr(), k.data_ptr(), v.data_ptr(),
                                     None if kv_valid_len is None else kv_valid_len.data_ptr(),
-                                    None if bv is None else ctypes.byref(bv), float(sm_scale), ws.data_ptr(), ws.numel(),
+                                    None if bv is None else ctypes.byref(bv), float(sm_scale), ws.data_ptr(), nbytes,
                                     o.data_ptr(), lse.data_ptr(), _lib.stream_int()), "lvx_attn_forward")
     _count(2)
 
 
-def attn_backward(do, q, k, v, o, lse, sm_scale, kv_valid_len, bias, scratch, dq, dk, dv) -> None:
-    """Its backward in one library call: delta, the cleared dQ accumulator (both in `scratch`, uint8), the block, and dQ
-    cast to its dtype. All tensors contiguous and checked by the caller."""
+def attn_backward(do, q, k, v, o, lse, sm_scale, kv_valid_len, bias, dq, dk, dv) -> None:
+    """Its backward in one library call: delta, the cleared dQ accumulator, the block, and dQ cast to its dtype. All
+    tensors contiguous and checked by the caller."""
     _require_cuda(do, q, k, v, o, lse, kv_valid_len)
     lib = _lib.load()
     if v.shape != k.shape or do.numel() != q.numel() or o.numel() != q.numel() or do.dtype != q.dtype or o.dtype != q.dtype:
@@ -236,11 +238,12 @@ def attn_backward(do, q, k, v, o, lse, sm_scale, kv_valid_len, bias, scratch, dq
     shp = shape_of(q, k)
     if kv_valid_len is not None and kv_valid_len.numel() != shp.B:
         raise ValueError("kv_valid_len must be an int32 tensor with one entry per batch element")
+    scratch = lse.new_empty(q.numel() + lse.numel())         # fp32 dQ and delta; the call's own, as in attn_forward
     bv, keep = _bias_view(bias, q, k) if bias is not None else (None, None)
     _lib.check(lib.lvx_attn_backward(ctypes.byref(shp), do.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(),
                                      o.data_ptr(), lse.data_ptr(), None if kv_valid_len is None else kv_valid_len.data_ptr(),
                                      None if bv is None else ctypes.byref(bv), float(sm_scale), scratch.data_ptr(),
-                                     scratch.numel(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _lib.stream_int()),
+                                     scratch.numel() * 4, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _lib.stream_int()),
                "lvx_attn_backward")
     _count(2 if q.dtype == torch.float32 else 3)
 

@@ -119,3 +119,59 @@ def test_a_pass_that_found_the_word_set_is_reported(cuda_device, dtype, bias):
     finally:
         lib.lvx_p2p_set_timeout(120.0)
         _lib.device_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_two_threads_on_two_streams(cuda_device, dtype):
+    """Scratch is a call's own: passes that two threads launch at the same time, each on its own stream, give what they give
+    one after the other (dQ up to the order of its additions)."""
+    import threading
+    shapes = [(1, 8, 2, 96, 3000), (2, 4, 2, 40, 1500)]
+    inputs = [[t.to(cuda_device) for t in orc.make_inputs(*s, 128, 85 + i, dtype)] for i, s in enumerate(shapes)]
+    alone = [both_passes(*x) for x in inputs]
+    torch.cuda.synchronize()
+    got = [[], []]
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(30):
+                got[i].append(both_passes(*inputs[i]))
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20
+    for i in range(2):
+        assert len(got[i]) == 30
+        for outs in got[i]:
+            for name, a, b in zip(("o", "lse", "dq", "dk", "dv"), outs, alone[i]):
+                if name == "dq":
+                    assert (a.float() - b.float()).abs().max() <= tol * b.float().abs().max()
+                else:
+                    assert torch.equal(a, b), name
+
+
+def test_captured_passes_keep_their_scratch(cuda_device):
+    """Passes captured into a graph, then larger ones outside of it, then the graph again with new inputs."""
+    q, k, v, do = (t.to(cuda_device) for t in orc.make_inputs(1, 8, 2, 50, 2000, 128, 87, torch.bfloat16))
+    both_passes(q, k, v, do)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs = both_passes(q, k, v, do)
+    big = [t.to(cuda_device) for t in orc.make_inputs(1, 8, 2, 700, 9000, 128, 88, torch.bfloat16)]
+    both_passes(*big)
+    for seed in (89, 90):
+        for old, new in zip((q, k, v, do), orc.make_inputs(1, 8, 2, 50, 2000, 128, seed, torch.bfloat16)):
+            old.copy_(new)
+        both_passes(*big)
+        graph.replay()
+        torch.cuda.synchronize()
+        want = both_passes(q, k, v, do)
+        for name, a, b in zip(("o", "lse", "dq", "dk", "dv"), outs, want):
+            if name == "dq":
+                assert (a.float() - b.float()).abs().max() <= 2.0 ** -8 * b.float().abs().max()
+            else:
+                assert torch.equal(a, b), name
