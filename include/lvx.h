@@ -186,7 +186,8 @@ int lvx_knorm_bwd(int dtype, const void* k, const void* dk, const float* rstd, c
 
 /* The gradients of the projection's outputs as its weight gradients want them: dk_rows, dv_rows [batch, S, Hkv, 128]
  * (one row per key) from dk, dv [batch, Hkv, S, 128], with the norm's backward applied to dk on the way as in
- * lvx_knorm_bwd (norm_w NULL: none; dw accumulates otherwise). The reference leaves this to autograd over its modules
+ * lvx_knorm_bwd (norm_w NULL: none; dw accumulates otherwise). Of dk_rows, dv_rows and dw those that are NULL are not made.
+ * The reference leaves this to autograd over its modules
  * (test_llama3.py:394-419). */
 int lvx_kv_project_grad_rows(int dtype, const void* k, const void* dk, const void* dv, const float* rstd,
                              const void* norm_w, void* dk_rows, void* dv_rows, float* dw, int batch, int Hkv, int S,

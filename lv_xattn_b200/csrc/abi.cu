@@ -476,10 +476,10 @@ int lvx_kv_project_grad_rows(int dtype, const void* k, const void* dk, const voi
   LVX_REQUIRE_PTR(dk, who);
   LVX_REQUIRE_PTR(dv, who);
   LVX_REQUIRE_PTR(rstd, who);
-  LVX_REQUIRE_PTR(dk_rows, who);
-  LVX_REQUIRE_PTR(dv_rows, who);
+  if (dk_rows) LVX_REQUIRE_PTR(dk_rows, who);
+  if (dv_rows) LVX_REQUIRE_PTR(dv_rows, who);
   if (norm_w) {
-    LVX_REQUIRE_PTR(dw, who);
+    if (dw) LVX_REQUIRE_PTR(dw, who);
     if (reinterpret_cast<uintptr_t>(norm_w) & 7u) return fail(LVX_ERR_ALIGN, "%s: norm_w is not 8-byte aligned", who);
   }
   return launch_kvproj_grad_rows(dtype, k, dk, dv, rstd, norm_w, dk_rows, dv_rows, dw, batch, Hkv, S,

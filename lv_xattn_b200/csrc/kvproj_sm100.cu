@@ -312,7 +312,8 @@ int launch_kv_project(int dtype, const void* x, const void* wk, const void* wv, 
 // what the kernel waited for. Measured on 8 heads x 51,232 keys (315 MB): 235 -> 68 us.
 // ROWS: the outputs are laid out [B, S, Hkv, 128], one row of Hkv * 128 columns per key, and dv is brought into the same
 // layout on the way: the weight gradients are then plain [Hkv*128, B*S] x [B*S, hidden] products, which the library runs in
-// 282 us a piece at 51,232 keys against 387 on the transposed head-major gradients (and a copy it makes of those).
+// 282 us a piece at 51,232 keys against 387 on the transposed head-major gradients (and a copy it makes of those). Outputs
+// that are NULL (the gradient of a frozen projection, or of its norm) are not made, nor is what only they need read.
 constexpr int KN_ROWS = 4;              // rows in flight per half-warp
 constexpr int KN_BLOCK_ROWS = 16 * KN_ROWS;
 
@@ -342,16 +343,19 @@ knorm_bwd_kernel(const void* __restrict__ k, const void* __restrict__ dk, const 
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) dwl[i] = 0.f;
+  const bool with_k = dkpre != nullptr || dw != nullptr, with_v = ROWS && dv_rows != nullptr;
   for (long base = long(blockIdx.x) * KN_BLOCK_ROWS; base < rows; base += long(gridDim.x) * KN_BLOCK_ROWS) {
     uint4 kk[KN_ROWS], gg[KN_ROWS], vv[ROWS ? KN_ROWS : 1];
     float rs[KN_ROWS];
 #pragma unroll
     for (int u = 0; u < KN_ROWS; ++u) {
       const long row = min(base + u * 16 + half, rows - 1);
-      kk[u] = reinterpret_cast<const uint4*>(k)[row * 16 + l16];
-      gg[u] = reinterpret_cast<const uint4*>(dk)[row * 16 + l16];
-      rs[u] = rstd[row];
-      if constexpr (ROWS) vv[u] = reinterpret_cast<const uint4*>(dv)[row * 16 + l16];
+      if (!ROWS || with_k) {
+        kk[u] = reinterpret_cast<const uint4*>(k)[row * 16 + l16];
+        gg[u] = reinterpret_cast<const uint4*>(dk)[row * 16 + l16];
+        rs[u] = rstd[row];
+      }
+      if (with_v) vv[ROWS ? u : 0] = reinterpret_cast<const uint4*>(dv)[row * 16 + l16];
     }
 #pragma unroll
     for (int u = 0; u < KN_ROWS; ++u) {
@@ -369,7 +373,8 @@ knorm_bwd_kernel(const void* __restrict__ k, const void* __restrict__ dk, const 
       if constexpr (ROWS) {
         const long slab = row / s_len, b = slab / hkv;               // (batch, head)
         out = (b * s_len + (row - slab * s_len)) * hkv + (slab - b * hkv);
-        reinterpret_cast<uint4*>(dv_rows)[out * 16 + l16] = vv[u];
+        if (with_v) reinterpret_cast<uint4*>(dv_rows)[out * 16 + l16] = vv[u];
+        if (!with_k) continue;
         if (norm_w == nullptr) {                                     // no norm: K = Kpre
           reinterpret_cast<uint4*>(dkpre)[out * 16 + l16] = gg[u];
           continue;
@@ -383,6 +388,7 @@ knorm_bwd_kernel(const void* __restrict__ k, const void* __restrict__ dk, const 
         o[i] = r * (wf[i] * gf[i] - xhat * mean);
         dwl[i] = fmaf(gf[i], xhat, dwl[i]);
       }
+      if (ROWS && dkpre == nullptr) continue;
       reinterpret_cast<uint4*>(dkpre)[out * 16 + l16] =
           make_uint4(kp_pack<IS_BF16>(o[0], o[1]), kp_pack<IS_BF16>(o[2], o[3]), kp_pack<IS_BF16>(o[4], o[5]),
                      kp_pack<IS_BF16>(o[6], o[7]));
@@ -395,7 +401,7 @@ knorm_bwd_kernel(const void* __restrict__ k, const void* __restrict__ dk, const 
     float a = 0.f;
 #pragma unroll
     for (int w = 0; w < 16; ++w) a += s_dw[w][threadIdx.x];
-    if (norm_w) atomicAdd(dw + threadIdx.x, a);
+    if (dw) atomicAdd(dw + threadIdx.x, a);
   }
 }
 
@@ -414,6 +420,8 @@ int launch_knorm_bwd(int dtype, const void* k, const void* dk, const float* rstd
 int launch_kvproj_grad_rows(int dtype, const void* k, const void* dk, const void* dv, const float* rstd, const void* norm_w,
                             void* dk_rows, void* dv_rows, float* dw, int batch, int hkv, int s, cudaStream_t st) {
   const long rows = long(batch) * hkv * s;
+  if (!norm_w) dw = nullptr;
+  if (!dk_rows && !dv_rows && !dw) return LVX_OK;
   const long blocks = std::min<long>((rows + KN_BLOCK_ROWS - 1) / KN_BLOCK_ROWS, 148 * 6);
   if (blocks == 0) return LVX_OK;
   const int* sp = device_status_ptr();

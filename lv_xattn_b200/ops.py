@@ -375,9 +375,9 @@ def knorm_bwd(k, dk, rstd, norm_weight):
     return dkpre, dw
 
 
-def kv_grad_rows(k, dk, dv, rstd, norm_weight):
+def kv_grad_rows(k, dk, dv, rstd, norm_weight, want_k=True, want_v=True, want_w=True):
     """The gradients of K and V as the projection's weight gradients want them: (dk_rows, dv_rows [B, S, Hkv*128], dw fp32
-    [128] or None), with the backward of the K norm applied to dk."""
+    [128]), with the backward of the K norm applied to dk. None for those that are not wanted, and for dw without a norm."""
     _require_cuda(k, dk, dv, rstd, norm_weight)
     lib = _lib.load()
     k, dk, dv, rstd = _contig(k), _contig(dk), _contig(dv), _contig(rstd)
@@ -386,14 +386,16 @@ def kv_grad_rows(k, dk, dv, rstd, norm_weight):
         raise ValueError("kv_grad_rows: k, dk, dv [B, Hkv, S, 128] in one 16-bit dtype and fp32 rstd with one entry per row")
     B, H, S, _ = k.shape
     w = _contig(norm_weight.to(k.dtype)) if norm_weight is not None else None
-    rows = torch.empty(2, B, S, H * 128, dtype=k.dtype, device=k.device)
-    dw = torch.zeros(128, dtype=torch.float32, device=k.device) if w is not None else None
+    dk_rows, dv_rows = (torch.empty(B, S, H * 128, dtype=k.dtype, device=k.device) if want else None for want in (want_k, want_v))
+    dw = torch.zeros(128, dtype=torch.float32, device=k.device) if w is not None and want_w else None
+    if dk_rows is None and dv_rows is None and dw is None:
+        return None, None, None
     _lib.check(lib.lvx_kv_project_grad_rows(_lib.dtype_code(k.dtype), k.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                                            rstd.data_ptr(), None if w is None else w.data_ptr(), rows[0].data_ptr(),
-                                            rows[1].data_ptr(), None if dw is None else dw.data_ptr(), B, H, S,
-                                            _lib.stream_int()), "lvx_kv_project_grad_rows")
+                                            rstd.data_ptr(), *(None if t is None else t.data_ptr()
+                                                               for t in (w, dk_rows, dv_rows, dw)),
+                                            B, H, S, _lib.stream_int()), "lvx_kv_project_grad_rows")
     _count()
-    return rows[0], rows[1], dw
+    return dk_rows, dv_rows, dw
 
 
 def fwd_merge_parts(o_parts, lse_parts, out_dtype, o_out=None, lse_out=None):

@@ -31,17 +31,18 @@ class KVProjectFunc(torch.autograd.Function):
     def backward(ctx, dk, dv):
         states, wk, wv, norm_weight, k, rstd = ctx.saved_tensors
         hid = states.shape[-1]
-        dk_rows, dv_rows, dnw = ops.kv_grad_rows(k, dk, dv, rstd, norm_weight)
-        dk_rows, dv_rows = dk_rows.flatten(0, 1), dv_rows.flatten(0, 1)          # [B*S, Hkv*128]
+        want_x, want_wk, want_wv, want_nw = ctx.needs_input_grad[:4]
+        dk_rows, dv_rows, dnw = ops.kv_grad_rows(k, dk, dv, rstd, norm_weight, want_x or want_wk, want_x or want_wv, want_nw)
+        dk_rows, dv_rows = (None if t is None else t.flatten(0, 1) for t in (dk_rows, dv_rows))      # [B*S, Hkv*128]
         g_wk = g_wv = g_states = g_nw = None
         x = states.reshape(-1, hid)
-        if ctx.needs_input_grad[1]:
+        if want_wk:
             g_wk = torch.mm(dk_rows.t(), x)
-        if ctx.needs_input_grad[2]:
+        if want_wv:
             g_wv = torch.mm(dv_rows.t(), x)
-        if ctx.needs_input_grad[0]:
+        if want_x:
             g_states = (torch.mm(dk_rows, wk) + torch.mm(dv_rows, wv)).view(states.shape)
-        if norm_weight is not None and ctx.needs_input_grad[3]:
+        if norm_weight is not None and want_nw:
             g_nw = dnw.to(norm_weight.dtype)
         return g_states, g_wk, g_wv, g_nw, None, None
 
