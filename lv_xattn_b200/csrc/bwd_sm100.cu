@@ -46,7 +46,8 @@
 // columns, low halves in the rest) and dS^T takes two shared-memory tiles, which leaves one buffer for dO instead of
 // two (dO of tile j is free after dV(j), so its successor still arrives under the dS^T half). dV, dK and dQ^T take
 // 16 MMAs instead of 8. The transposed frame suits the bias: a warp's lanes are 32 consecutive keys, so a column's bias
-// values are one 128-byte read. fp16 stays with the general kernel: dS has no bound there, and half of it could
+// values are one 128-byte read. An infinity in dO times the low half of P, which may be zero or negative, is NaN where
+// the plain product is infinite: a key whose dV holds NaN is made again without halves (plain_dv). fp16 stays with the general kernel: dS has no bound there, and half of it could
 // fall among fp16's subnormals. Measured at 32 heads, 512 x 6,404: 330 us (436 with half of the bias requested late,
 // at 72 registers; 5,177 on the FP32-FMA kernel that this form replaced).
 #include "lvx_internal.h"
@@ -120,8 +121,27 @@ struct BwdParams {
   int accumulate;      // 0 overwrite fp32, 1 add to fp32, 2 write the finished gradient in the input dtype
   BlockWait bw;        // query blocks that may still be arriving from other ranks
   BiasView bias;       // BIAS kernel only
+  const void *q, *d_o, *k;      // BIAS: for plain_dv
   int* status;
 };
+
+// 32 columns of one key's dV over all query rows of its slab, as plain fp32 sums. `bias` points at this batch entry's, KV
+// head's and key's first value; q, d_o and lse start at the slab in the first query block, blk_rows rows before the next.
+template <bool IS_BF16>
+__device__ __noinline__ void plain_dv(float* dv, const uint16_t* k, const uint16_t* q, const uint16_t* d_o, const float* lse,
+                                      const float* bias, long long s_blk, long long s_h, long long s_q, int sq, int rows,
+                                      int nblk, size_t blk_rows, float c) {
+  for (int i = 0; i < 32; ++i) dv[i] = 0.f;
+  for (int blk = 0; blk < nblk; ++blk)
+    for (int row = 0; row < rows; ++row) {
+      const size_t at = blk * blk_rows + row;
+      float l2 = lse[at] * 1.4426950408889634f;
+      if (l2 == -INFINITY) l2 = INFINITY;
+      const float b = bias[blk * s_blk + (row / sq) * s_h + (row % sq) * s_q];
+      const float s = fmaf(b, 1.4426950408889634f, dot128<IS_BF16>(k, q + at * 128) * c);
+      axpy32<IS_BF16>(dv, ex2f(s - l2), d_o + at * 128);
+    }
+}
 
 // Development aid, compiled only with -DLVX_DEV_STAMPS (never in the shipped library): cycle stamps of CTA
 // (0,0), tiles 4..11, 16 slots per tile and role, printed by the launcher.
@@ -430,6 +450,25 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             tmem_ld32(tmem_base + (which ? TM_DV : TM_DK) + lane_sel + cg * 32, a);
             tc_wait_ld();
             const float mul = which ? 1.f : p.scale;
+            if constexpr (BIAS) {
+              float sum = 0.f;
+#pragma unroll
+              for (int i = 0; i < 32; ++i) sum += __uint_as_float(a[i]);
+              if (which && row_valid && isnan(sum)) {
+                float again[32];
+                const size_t at = size_t(I.slab) * p.rows;
+                plain_dv<IS_BF16>(again, static_cast<const uint16_t*>(p.k) + (size_t(I.slab) * p.skv + I.kv0 + r) * 128,
+                                  static_cast<const uint16_t*>(p.q) + at * 128,
+                                  static_cast<const uint16_t*>(p.d_o) + at * 128 + cg * 32, p.lse + at,
+                                  p.bias.base + (I.slab / p.hkv) * p.bias.s_b + (I.slab % p.hkv) * p.bias.g * p.bias.s_h +
+                                      (I.kv0 + r) * p.bias.s_kv,
+                                  p.bias.s_blk, p.bias.s_h, p.bias.s_q, p.bias.sq, p.rows, p.nblk,
+                                  size_t(p.kv_slabs) * p.rows, c);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) a[i] = __float_as_uint(again[i]);
+              }
+              __syncwarp();
+            }
             if (ok_row && p.accumulate == 2) {
               uint4* d16 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(which ? p.dv_acc : p.dk_acc) + off);
 #pragma unroll
@@ -788,6 +827,9 @@ int launch_bwd_block(const lvx_shape& s, const void* q, const void* d_o, const f
   p.status = status;
   p.bw = make_block_wait(bw, qb);
   p.bias = make_bias(s, bias);
+  p.q = q;
+  p.d_o = d_o;
+  p.k = k;
 
   p.kv_tiles = (s.Skv + 127) / 128;
   p.nitems = p.kv_tiles * p.kv_slabs;

@@ -66,6 +66,7 @@ struct FwdParams {
   float* ml_part;       // [B*Hkv][nsplit][rows][2]
   BlockWait bw;         // query blocks that may still be arriving from other ranks
   BiasView bias;        // additive bias (BIAS kernels only)
+  const void *q, *k, *v;                          // BIAS: for plain_values
   int bias_vec;         // its rows can be read 16 bytes at a time
   int* status;
 };
@@ -92,8 +93,22 @@ __device__ long long g_fwd_ts[3 * 8 * 8];
 // of its own row, which read directly would touch 32 lines a load; each warp therefore copies 32 rows x 32 keys at a time,
 // a row's 128 bytes by eight lanes, into a swizzled buffer of its own, two pieces ahead of the one it adds (rows that
 // are not 16-byte aligned, and the ragged last tile, are read directly). V keeps one stage then: its successor has the
-// whole softmax to arrive in. Measured at 32 heads, 512 x 6,404, bf16: 158 us (202 with direct reads, 2,154 on the
+// whole softmax to arrive in. An infinity in V times the second half of P, which may be zero or negative, is NaN where the
+// plain product is infinite: a row that ends with NaN although its sum is finite is made again without halves
+// (plain_values; nothing else pays for it). Measured at 32 heads, 512 x 6,404, bf16: 158 us (202 with direct reads, 2,154 on the
 // FP32-FMA kernel that this form replaced).
+
+// 32 columns of one row's O over keys [key0, key1), as plain fp32 sums.
+template <bool IS_BF16>
+__device__ __noinline__ void plain_values(float* o, const uint16_t* q, const uint16_t* k, const uint16_t* v, const float* bias,
+                                          long long s_kv, int key0, int key1, float c, float m) {
+  for (int i = 0; i < 32; ++i) o[i] = 0.f;
+  for (int key = key0; key < key1; ++key) {
+    const float s = fmaf(bias[key * s_kv], 1.4426950408889634f, dot128<IS_BF16>(q, k + size_t(key) * 128) * c);
+    axpy32<IS_BF16>(o, ex2f(s - m), v + size_t(key) * 128);
+  }
+}
+
 template <bool IS_BF16, bool BIAS>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -435,6 +450,22 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           uint32_t o[32];
           tmem_ld32(tO + q * 32, o);
           tc_wait_ld();
+          if constexpr (BIAS) {
+            float sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) sum += __uint_as_float(o[i]);
+            if (row < p.rows && isnan(sum) && l < INFINITY) {
+              float again[32];
+              const uint16_t* kv0 = static_cast<const uint16_t*>(p.k) + size_t(kvs) * p.skv * 128;
+              const uint16_t* vv0 = static_cast<const uint16_t*>(p.v) + size_t(kvs) * p.skv * 128;
+              plain_values<IS_BF16>(again, static_cast<const uint16_t*>(p.q) + (size_t(bh) * p.rows + row) * 128, kv0,
+                                    vv0 + q * 32, brow, p.bias.s_kv, tile0 * 128, min(valid, (tile0 + n) * 128), c,
+                                    m == -INFINITY ? 0.f : m);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(again[i]);
+            }
+            __syncwarp();
+          }
           if (row < p.rows) {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
@@ -683,6 +714,9 @@ int launch_fwd_block(const lvx_shape& s, const FwdPlan& pl, const void* q, const
   p.status = status;
   p.bw = make_block_wait(bw, qb);
   p.bias = make_bias(s, bias);
+  p.q = q;
+  p.k = k;
+  p.v = v;
   p.bias_vec = bias && bias->stride_kv == 1 && (reinterpret_cast<uintptr_t>(bias->bias) & 15) == 0 &&
                ((bias->stride_block | bias->stride_b | bias->stride_h | bias->stride_q) & 3) == 0;
 

@@ -346,6 +346,38 @@ __device__ __forceinline__ void publish_status(const int* status) {
     __threadfence_system();
   }
 }
+// Product of two 128-wide 16-bit rows in fp32.
+template <bool IS_BF16>
+__device__ __forceinline__ float dot128(const void* a, const void* b) {
+  float s = 0.f;
+#pragma unroll 4
+  for (int i = 0; i < 16; ++i) {
+    const uint4 x = reinterpret_cast<const uint4*>(a)[i], y = reinterpret_cast<const uint4*>(b)[i];
+    const uint32_t u[4] = {x.x, x.y, x.z, x.w}, w[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = unpack16x2<IS_BF16>(u[e]), g = unpack16x2<IS_BF16>(w[e]);
+      s = fmaf(f.x, g.x, s);
+      s = fmaf(f.y, g.y, s);
+    }
+  }
+  return s;
+}
+// acc[0..31] += w * row[0..31] (16-bit)
+template <bool IS_BF16>
+__device__ __forceinline__ void axpy32(float* acc, float w, const void* row) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint4 x = reinterpret_cast<const uint4*>(row)[i];
+    const uint32_t u[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = unpack16x2<IS_BF16>(u[e]);
+      acc[8 * i + 2 * e] = fmaf(w, f.x, acc[8 * i + 2 * e]);
+      acc[8 * i + 2 * e + 1] = fmaf(w, f.y, acc[8 * i + 2 * e + 1]);
+    }
+  }
+}
 // Two fp32 lanes per instruction (sm_100 packed arithmetic): halves the issue slots of the softmax inner loops.
 __device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
   uint64_t r;

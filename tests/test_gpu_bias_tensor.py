@@ -135,3 +135,38 @@ def test_small_probabilities_beside_a_dominant_key(cuda_device, dtype, below, at
     err = ((o.cpu().double() - ref).norm() / ref.norm()).item()
     assert err <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10), err
     assert (lse.cpu().double() - torch.logsumexp(bias.double()[0, 0], -1)).abs().max() <= 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_infinite_values_and_gradients(cuda_device, dtype):
+    """An infinite V gives its column of O, and an infinite dO its column of dV, the infinity that a plain sum gives them, and
+    NaN stays in its column: the second part of P, which may be zero or negative, must not turn them into NaN. A -inf key
+    is no key."""
+    from lv_xattn_b200 import ops
+    B, Hq, Hkv, Sq, Skv = 1, 4, 2, 150, 700
+    q, k, v, do = orc.make_inputs(B, Hq, Hkv, Sq, Skv, 128, 78, dtype)
+    q[..., 0] = q[..., 0].abs() + 0.125
+    k[0, 1, 400, 0] = float("-inf")
+    v[0, 0, 3, 5] = float("inf")
+    v[0, 0, 690, 6] = float("-inf")
+    v[0, 1, 301, 7] = float("nan")
+    do[0, 1, 20, 8] = float("inf")
+    do[0, 2, 149, 9] = float("-inf")
+    do[0, 3, 40, 10] = float("nan")
+    bias = torch.randn(1, 1, Sq, Skv, generator=torch.Generator().manual_seed(79))
+    k6, v6 = (t.double().repeat_interleave(2, 1) for t in (k, v))
+    p6 = (q.double() @ k6.transpose(-1, -2) * SCALE + bias.double()).softmax(-1)
+    o6 = p6 @ v6
+    dv6 = (p6.transpose(-1, -2) @ do.double()).view(1, 2, 2, Skv, 128).sum(2)
+    qd, kd, vd, dod, bd = (t.to(cuda_device) for t in (q, k, v, do, bias))
+    o, lse = ops.fwd_block(qd, kd, vd, SCALE, bias=bd)
+    dq = torch.zeros(B, Hq, Sq, 128, device=cuda_device)
+    dk, dv = torch.empty_like(kd), torch.empty_like(vd)
+    ops.bwd_block(qd, dod, lse, torch.zeros(B * Hq, Sq, device=cuda_device), kd, vd, SCALE, dq, dk, dv, "final", bias=bd)
+    dv[0, 1, 400] = dv6[0, 1, 400] = 0       # no key: 0 * inf there
+    for name, got, ref in (("o", o, o6), ("dv", dv, dv6)):
+        got = got.double().cpu()
+        for at in (torch.isnan, torch.isposinf, torch.isneginf):
+            assert torch.equal(at(got), at(ref)), (name, at.__name__)
+        fin = torch.isfinite(ref)
+        assert ((got - ref)[fin].norm() / ref[fin].norm()).item() <= 1e-2, name
