@@ -438,6 +438,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         if (lane == 0) mbar_arrive(&bars[FB_P_FULL + wg]);
         if ((warp & 3) == 0) FWD_TS(wg, 4);
       }
+      // a warp that gave up inside the loop has pieces of the bias on their way
+      if (BIAS) asm volatile("cp.async.wait_all;" ::: "memory");
       // ------------------------------- epilogue -------------------------------
       const int row = mb * 256 + wg * 128 + row_in_tile;
       if (alive) alive = mbar_wait(&bars[FB_O_DONE + wg], 0, abort_flag, p.status, FWD_CODE(wg, FB_O_DONE), p.bw.pipe_limit);
