@@ -790,11 +790,8 @@ int launch_bwd_block(const lvx_shape& s, const void* q, const void* d_o, const f
   if (accumulate_dkdv < 0 || accumulate_dkdv > 2)
     return fail(LVX_ERR_SHAPE, "lvx_bwd_block: accumulate_dkdv must be 0, 1 or 2 (got %d)", accumulate_dkdv);
   // bias: the tensor-core form takes bf16 (see the head of this file)
-  if (bias && s.dtype != LVX_BF16)
+  if (s.dtype == LVX_FP32 || (bias && s.dtype != LVX_BF16))
     return launch_bwd_block_general(s, q, d_o, lse, delta, k, v, kv_valid_len, bias, sm_scale, dq_acc, dk_acc, dv_acc,
-                                 accumulate_dkdv, st);
-  if (s.dtype == LVX_FP32)
-    return launch_bwd_block_fp32(s, q, d_o, lse, delta, k, v, kv_valid_len, sm_scale, dq_acc, dk_acc, dv_acc,
                                  accumulate_dkdv, st);
   const int g = s.Hq / s.Hkv;
   const int rows = g * s.Sq;

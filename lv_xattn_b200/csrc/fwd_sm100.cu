@@ -681,8 +681,7 @@ int launch_fwd_block(const lvx_shape& s, const FwdPlan& pl, const void* q, const
                      const int32_t* kv_valid_len, float sm_scale, float* o_part, float* ml_part, int* status,
                      cudaStream_t st, const lvx_block_wait* bw, const lvx_bias* bias) {
   if (!(sm_scale > 0.f)) return fail(LVX_ERR_SHAPE, "lvx_fwd_block: sm_scale must be positive");
-  if (s.dtype == LVX_FP32 && bias) return launch_fwd_block_general(s, pl, q, k, v, kv_valid_len, bias, sm_scale, o_part, ml_part, st);
-  if (s.dtype == LVX_FP32) return launch_fwd_block_fp32(s, pl, q, k, v, kv_valid_len, sm_scale, o_part, ml_part, st);
+  if (s.dtype == LVX_FP32) return launch_fwd_block_general(s, pl, q, k, v, kv_valid_len, bias, sm_scale, o_part, ml_part, st);
   if (pl.rows <= kFewRows && q_blocks_of(s) == 1 && bw == nullptr && bias == nullptr)
     return launch_fwd_rows(s, pl, q, k, v, kv_valid_len, sm_scale, o_part, ml_part, status, st);
   CUtensorMap tmQ, tmK, tmV;

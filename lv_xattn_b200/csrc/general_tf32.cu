@@ -126,22 +126,18 @@ __device__ __forceinline__ void mma3x4(float (*acc)[4], const AFrag<EXA, CLAMP>&
       if (EXB) s[n][i].hi = __float_as_uint(b(n, i));
       else s[n][i] = split_tf32<CLAMP>(b(n, i));
     }
-  if constexpr (EXA && EXB) {
+  static_assert(EXB || !EXA, "an exact A comes with an exact B");
+  if constexpr (EXA) {
 #pragma unroll
     for (int n = 0; n < 4; ++n) mma_tf32(t[n], a.hi, s[n][0].hi, s[n][1].hi, zero);
   } else {
-    if constexpr (!EXA) {
-      // an exact B keeps its infinities in hi; they belong to the product with A's hi alone
-      auto beside_lo = [](uint32_t hi) { return EXB && CLAMP ? clamp_tf32(hi) : hi; };
+    // an exact B keeps its infinities in hi; they belong to the product with A's hi alone
+    auto beside_lo = [](uint32_t hi) { return EXB && CLAMP ? clamp_tf32(hi) : hi; };
 #pragma unroll
-      for (int n = 0; n < 4; ++n) mma_tf32(t[n], a.lo, beside_lo(s[n][0].hi), beside_lo(s[n][1].hi), zero);
-    }
+    for (int n = 0; n < 4; ++n) mma_tf32(t[n], a.lo, beside_lo(s[n][0].hi), beside_lo(s[n][1].hi), zero);
     if constexpr (!EXB) {
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        if constexpr (EXA) mma_tf32(t[n], a.hi, s[n][0].lo, s[n][1].lo, zero);
-        else mma_tf32(t[n], a.hi, s[n][0].lo, s[n][1].lo, t[n]);
-      }
+      for (int n = 0; n < 4; ++n) mma_tf32(t[n], a.hi, s[n][0].lo, s[n][1].lo, t[n]);
     }
 #pragma unroll
     for (int n = 0; n < 4; ++n) mma_tf32(t[n], a.hi, s[n][0].hi, s[n][1].hi, t[n]);
@@ -593,18 +589,6 @@ int launch_bwd_block_general(const lvx_shape& s, const void* q, const void* d_o,
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "fp32 bwd kernel launch");
   return LVX_OK;
-}
-
-int launch_fwd_block_fp32(const lvx_shape& s, const FwdPlan& pl, const void* q, const void* k, const void* v,
-                          const int32_t* kv_valid_len, float sm_scale, float* o_part, float* ml_part, cudaStream_t st) {
-  return launch_fwd_block_general(s, pl, q, k, v, kv_valid_len, nullptr, sm_scale, o_part, ml_part, st);
-}
-
-int launch_bwd_block_fp32(const lvx_shape& s, const void* q, const void* d_o, const float* lse, const float* delta,
-                          const void* k, const void* v, const int32_t* kv_valid_len, float sm_scale, float* dq_acc,
-                          float* dk_acc, float* dv_acc, int accumulate_dkdv, cudaStream_t st) {
-  return launch_bwd_block_general(s, q, d_o, lse, delta, k, v, kv_valid_len, nullptr, sm_scale, dq_acc, dk_acc, dv_acc,
-                               accumulate_dkdv, st);
 }
 
 }  // namespace lvx

@@ -79,13 +79,8 @@ int launch_bwd_block(const lvx_shape& s, const void* q, const void* d_o, const f
                      const lvx_block_wait* bw = nullptr, const lvx_bias* bias = nullptr);
 // Limit of the in-kernel waits for a peer's flag, in SM cycles (lvx_p2p_set_timeout).
 long long p2p_wait_limit_cycles();
-// fp32 inputs (general_tf32.cu; same workspace layout and masking rules as the 16-bit path)
-int launch_fwd_block_fp32(const lvx_shape& s, const FwdPlan& p, const void* q, const void* k, const void* v,
-                          const int32_t* kv_valid_len, float sm_scale, float* o_part, float* ml_part, cudaStream_t st);
-int launch_bwd_block_fp32(const lvx_shape& s, const void* q, const void* d_o, const float* lse, const float* delta,
-                          const void* k, const void* v, const int32_t* kv_valid_len, float sm_scale, float* dq_acc,
-                          float* dk_acc, float* dv_acc, int accumulate_dkdv, cudaStream_t st);
-// The general block kernels: fp32 (forward) and fp32 or fp16 (backward), optional dense additive bias.
+// The general block kernels (general_tf32.cu; same workspace layout and masking rules as the 16-bit path): fp32 (forward)
+// and fp32 or fp16 (backward), optional dense additive bias.
 int launch_fwd_block_general(const lvx_shape& s, const FwdPlan& p, const void* q, const void* k, const void* v,
                           const int32_t* kv_valid_len, const lvx_bias* bias, float sm_scale, float* o_part,
                           float* ml_part, cudaStream_t st);
