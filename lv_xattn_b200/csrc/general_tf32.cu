@@ -8,7 +8,7 @@
 // fp32 accumulator by the FMA pipe, so the long sums keep fp32's own rounding (and take a sixteenth of the additions that a
 // plain FMA loop takes: the error against 64 bits at 512 x 8,192 is 5.9e-7 where an FMA loop's was 1.1e-6). 16-bit
 // inputs are exact in tf32 and take no lo.
-// Measured at 32 heads, 512 x 8,192: forward 2.47 -> 1.42 ms, backward 5.84 -> 3.62 ms.
+// Measured at 32 heads, 512 x 8,192: forward 2.47 -> 1.34 ms, backward 5.84 -> 3.65 ms.
 // What bounds it: mma.sync runs tf32 at 484 FMA/clk/SM here, i.e. 161 a clock for three products, against 128 (with
 // packed arithmetic, 104 without) on the FMA pipe, where moreover every operand of a register tile has to come through
 // shared memory at 4 bytes a lane and clock: the FMA kernels that this replaces sat at 48. tcgen05 is not used: it takes
@@ -75,9 +75,9 @@ __device__ __forceinline__ uint32_t clamp_tf32(uint32_t x) {
 // largest float rounding gives infinity, and lo the other one; every product with such a value, or with an infinite one,
 // is then NaN. With CLAMP hi is always finite: near the largest float lo takes the rest, and for an infinite x (or NaN) lo
 // is x, so that lo*b is what x*b is and nothing of the other sign or NaN is added to it.
-// A CTA walks over its tiles without CLAMP first, and again with it where NaN came out: 512 x 8,192 takes 5.09 ms forward and
-// backward (5.05 without any of this), against 5.33 with the clamp in every split and 5.26 with a look at the values of
-// every tile as it arrives. A result that is NaN by right takes both walks.
+// A CTA walks over its tiles without CLAMP first, and again with it where NaN came out: of 512 x 8,192, forward and
+// backward, that takes 0.7 %, against 5.7 % with the clamp in every split and 4 % with a look at the values of every tile
+// as it arrives. A result that is NaN by right takes both walks.
 struct Split {
   uint32_t hi, lo;
 };
@@ -193,6 +193,10 @@ struct Fp32FwdParams {
 // the warp that made them.
 constexpr int GF_SMEM = (128 * GT_LD + 4 * GT_TILE) * sizeof(float);
 
+// BIAS: a thread's 32 values of a tile are all requested before the products, under which they arrive. Requested one by one
+// between the products and the softmax they took nearly as long as the products: 32 slabs of 130 rows x 1,601 keys 289 -> 188
+// us (168 without a bias), 8 slabs of 160 rows x 6,404 keys 196 -> 160. Without a bias the kernel carries none of it.
+template <bool BIAS>
 __global__ void __launch_bounds__(256, 1)
 fp32_fwd_kernel(const Fp32FwdParams p) {
   if (p.status && *reinterpret_cast<const volatile int*>(p.status) != 0) return;
@@ -209,10 +213,10 @@ fp32_fwd_kernel(const Fp32FwdParams p) {
   const float* ks = p.k + size_t(kvs) * p.skv * 128;
   const float* vs = p.v + size_t(kvs) * p.skv * 128;
   const int row0 = mb * 128 + warp * 16 + g;  // fragment rows row0, row0 + 8
-  const float* brow[2];
+  const float* brow[2];                       // (rows that do not exist: the last one's)
 #pragma unroll
   for (int i = 0; i < 2; ++i)
-    brow[i] = row0 + 8 * i < p.rows ? bias_row(p.bias, slab, kvs, p.kv_slabs, p.hkv, row0 + 8 * i) : nullptr;
+    brow[i] = BIAS ? bias_row(p.bias, slab, kvs, p.kv_slabs, p.hkv, min(row0 + 8 * i, p.rows - 1)) : nullptr;
 
   float m[2], l[2], o[16][4];
   // the walk over the keys; a second one with CLAMP where NaN came out
@@ -240,11 +244,15 @@ fp32_fwd_kernel(const Fp32FwdParams p) {
       const float* tile = sKV + 2 * st * GT_TILE;
       const float* kb = tile + g * GT_LD + t;
       const float* vb = tile + GT_TILE + 2 * t * GT_LD + g;
+      float bv[BIAS ? 8 : 1][4];
+      if constexpr (BIAS) {
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) bv[n][e] = __ldg(brow[e >> 1] + min(kv0 + n * 8 + 2 * t + (e & 1), kv_end - 1) * p.bias.s_kv);
+      }
       float s[8][4];
-#pragma unroll
-      for (int n = 0; n < 8; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
+      set_zero(s);
 #pragma unroll 2
       for (int d = 0; d < 128; d += 8) {
         AFrag<false, cl.value> a;
@@ -263,7 +271,7 @@ fp32_fwd_kernel(const Fp32FwdParams p) {
           float sc = -INFINITY;
           if (col < kv_end) {
             sc = s[n][e] * p.scale_log2;
-            if (brow[i]) sc = fmaf(brow[i][col * p.bias.s_kv], 1.4426950408889634f, sc);   // scale*q.k + bias, base 2
+            if constexpr (BIAS) sc = fmaf(bv[n][e], 1.4426950408889634f, sc);              // scale*q.k + bias, base 2
           }
           s[n][e] = sc;
           mx[i] = fmaxf(mx[i], sc);
@@ -544,8 +552,13 @@ int launch_fwd_block_general(const lvx_shape& s, const FwdPlan& pl, const void* 
   p.ml_part = ml_part;
   p.status = device_status_ptr();
   dim3 grid(pl.m_blocks, q_blocks_of(s) * s.B * s.Hkv, pl.nsplit);
-  cudaError_t e = cudaFuncSetAttribute(fp32_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GF_SMEM);
-  if (e == cudaSuccess) fp32_fwd_kernel<<<grid, 256, GF_SMEM, st>>>(p);
+  cudaError_t e = cudaSuccess;
+  auto go = [&](auto kern) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GF_SMEM);
+    if (e == cudaSuccess) kern<<<grid, 256, GF_SMEM, st>>>(p);
+  };
+  if (bias) go(fp32_fwd_kernel<true>);
+  else go(fp32_fwd_kernel<false>);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(fp32 fwd)");
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "fp32 fwd kernel launch");
