@@ -213,6 +213,7 @@ fp32_fwd_kernel(const Fp32FwdParams p) {
   const float* ks = p.k + size_t(kvs) * p.skv * 128;
   const float* vs = p.v + size_t(kvs) * p.skv * 128;
   const int row0 = mb * 128 + warp * 16 + g;  // fragment rows row0, row0 + 8
+  const bool has_rows = mb * 128 + warp * 16 < p.rows;      // a warp without any only loads: its share of the CTA stays free
   const float* brow[2];                       // (rows that do not exist: the last one's)
 #pragma unroll
   for (int i = 0; i < 2; ++i)
@@ -241,6 +242,10 @@ fp32_fwd_kernel(const Fp32FwdParams p) {
       cp_commit();                               // possibly empty: the group before it is then complete after cp_wait<1>
       cp_wait<1>();
       __syncthreads();
+      if (!has_rows) {
+        __syncthreads();
+        continue;
+      }
       const float* tile = sKV + 2 * st * GT_TILE;
       const float* kb = tile + g * GT_LD + t;
       const float* vb = tile + GT_TILE + 2 * t * GT_LD + g;
