@@ -40,6 +40,8 @@
 //               per 60-75 cycles, so eight warps are needed)
 //   warp  24    TMA producer: K,V once; Q,dO tiles through a 2-stage ring
 //   warp  25    tcgen05.mma issuer; owns the TMEM allocation
+// (The BIAS form has 704 threads with 80 registers: four drain warps, 16-19, which take both column halves in turn; its
+// tiles last long enough for that.)
 //
 // The BIAS form (dense additive fp32 bias on the scores, bf16 inputs) keeps P and dS as the sum of two bf16 numbers:
 // both were fp32 before this path used the tensor core. P^T then fills X completely (high halves in its first 64
@@ -47,9 +49,10 @@
 // two (dO of tile j is free after dV(j), so its successor still arrives under the dS^T half). dV, dK and dQ^T take
 // 16 MMAs instead of 8. The transposed frame suits the bias: a warp's lanes are 32 consecutive keys, so a column's bias
 // values are one 128-byte read. An infinity in dO times the low half of P, which may be zero or negative, is NaN where
-// the plain product is infinite: a key whose dV holds NaN is made again without halves (plain_dv). fp16 stays with the general kernel: dS has no bound there, and half of it could
-// fall among fp16's subnormals. Measured at 32 heads, 512 x 6,404: 330 us (436 with half of the bias requested late,
-// at 72 registers; 5,177 on the FP32-FMA kernel that this form replaced).
+// the plain product is infinite: a key whose dV holds NaN is made again without halves (plain_dv). fp16 stays with the
+// general kernel: dS has no bound there, and half of it could fall among fp16's subnormals. Measured at 32 heads, 512 x
+// 6,404: 330 us (436 with half of the bias requested late, at 72 registers; 5,177 on the FP32-FMA kernel that this form
+// replaced). fp32 results against 64 bits: 2e-6 to 4e-6 (4e-7 to 8e-7 on that kernel).
 #include "lvx_internal.h"
 #include "sm100_prims.cuh"
 #include "block_wait.cuh"
@@ -74,7 +77,7 @@ constexpr int BWD_OFF_STAT = BWD_OFF_DS + BWD_TILE;              // [2][lse2 128
 constexpr int BWD_OFF_BAR = BWD_OFF_STAT + 2 * 256 * 4;
 constexpr int BWD_SMEM = BWD_OFF_BAR + 256;
 constexpr int BWD_COMPUTE_WARPS = 16;
-// BIAS: four drain warps (dQ^T in two halves each), so that a thread has 88 registers and the bias of a whole tile can be
+// BIAS: four drain warps (dQ^T in two halves each), so that a thread has 80 registers and the bias of a whole tile can be
 // on its way while S^T is
 constexpr int bwd_drain_warps(bool bias) { return bias ? 4 : 8; }
 constexpr int bwd_threads(bool bias) { return (BWD_COMPUTE_WARPS + bwd_drain_warps(bias) + 2) * 32; }

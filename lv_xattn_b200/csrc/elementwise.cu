@@ -3,7 +3,7 @@
 //   bwd_prep_kernel     delta = rowsum(O * dO)
 //   add_cast_kernel     out = cast(a + b)
 // A row of 128 values is read by one warp (fp32) or half a warp (16 bits), 16 bytes a lane, so that every access is a full
-// coalesced 512- or 256-byte row.
+// coalesced 512- or 256-byte row. Where rows are few, eight warps share one in the combine.
 #include "lvx_internal.h"
 #include "sm100_prims.cuh"
 #include <cuda_bf16.h>

@@ -8,9 +8,16 @@
 // rows merge once, at the end of the CTA's key range. The legacy mma.sync form is used on purpose: its operands come
 // from and go to registers, so the scores never leave the warp, and at <= 64 rows its rate is not what bounds the call.
 // K and V tiles are the same 128-byte-swizzled boxes as in the 256-row kernel and are read with conflict-free ldmatrix.
-// Measured: one token, 32 heads on 8 KV heads, 409,856 keys (1.68 GB of K and V): 447 -> 270 us a call, block and combine
-// together, i.e. 6.2 TB/s against a copy's 6.5. The line is at 64 rows because a fourth row group is where the mma work of
-// a tile (about 2,000 cycles) nears the time its bytes take (2,700).
+// Measured: one token, 32 heads on 8 KV heads, 409,856 keys (1.68 GB of K and V): 427-449 -> 249-252 us a call, block and
+// combine together, i.e. 6.7 TB/s (a copy reaches 6.5).
+// The line at 64 rows, block and combine in us, 256-row kernel -> this one, at 1 / 32 / 33 / 64 rows per KV head:
+//    8 KV heads x    300 keys    10.1 ->   5.9    11.0 ->   8.1    11.3 ->   8.7    11.5 ->   9.7
+//    8 KV heads x  6,404 keys    21.7 ->  11.1    21.9 ->  12.8    22.0 ->  15.3    21.6 ->  17.2
+//    8 KV heads x 102,464 keys   99.0 ->  66.2    99.3 ->  69.5    98.7 ->  93.8    98.0 ->  96.1
+//  128 KV heads x  1,601 keys    37.0 ->  22.2    37.2 ->  25.4    37.6 ->  34.5    40.0 ->  36.6
+//  128 KV heads x  6,404 keys   105.8 ->  64.6   106.2 ->  69.0   106.2 -> 105.6   108.6 -> 107.5
+// Up to 32 rows the call runs at the rate of its bytes; with 64 the mma work of a tile takes longer than they do, and where
+// the grid is large both kernels are even. More rows would be slower here than there.
 // The partials have the layout of that kernel, so the combine kernel does not care which of the two ran.
 #include "lvx_internal.h"
 #include "sm100_prims.cuh"

@@ -1,5 +1,6 @@
-"""The general block kernels with a dense additive bias (the reference's bias_func protocol, lv_xattn/attn.py:386-389:
-S = sm_scale*q.k + bias) through the C ABI, for every input dtype, against the CPU oracle. 16-bit tolerances as in the
+"""The block kernels with a dense additive bias (the reference's bias_func protocol, lv_xattn/attn.py:386-389:
+S = sm_scale*q.k + bias) through the C ABI, for every input dtype (fp32 and the fp16 backward
+run the general kernels, the others the tensor-core forms), against the CPU oracle. 16-bit tolerances as in the
 other tests (2e-2 max-abs, lse 1e-3, plus the relative criteria); fp32 1e-4."""
 import math
 
