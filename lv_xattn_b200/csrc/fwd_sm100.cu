@@ -67,7 +67,7 @@ struct FwdParams {
   BlockWait bw;         // query blocks that may still be arriving from other ranks
   BiasView bias;        // additive bias (BIAS kernels only)
   const void *q, *k, *v;                          // BIAS: for plain_values
-  int bias_vec;         // its rows can be read 16 bytes at a time
+  int bias_adjacent;    // neighbouring keys are neighbours in memory
   int* status;
 };
 
@@ -88,15 +88,17 @@ __device__ long long g_fwd_ts[3 * 8 * 8];
 
 // BIAS: a dense additive fp32 bias on the scores (S = scale * q.k + bias). P is then handed to the tensor core as the sum
 // of two 16-bit numbers (the second P V product costs 8 more MMAs per tile), which keeps 16 (bf16) or 22 (fp16, but
-// nothing below 2^-36 of the row's maximum) bits of it: the probabilities of this path were fp32 before it used the tensor core, and one 16-bit rounding would show. Every
-// tile takes the exact path, since scores that jump to -inf are what a bias is for. A thread needs 128 consecutive values
-// of its own row, which read directly would touch 32 lines a load; each warp therefore copies 32 rows x 32 keys at a time,
-// a row's 128 bytes by eight lanes, into a swizzled buffer of its own, two pieces ahead of the one it adds (rows that
-// are not 16-byte aligned, and the ragged last tile, are read directly). V keeps one stage then: its successor has the
-// whole softmax to arrive in. An infinity in V times the second half of P, which may be zero or negative, is NaN where the
-// plain product is infinite: a row that ends with NaN although its sum is finite is made again without halves
-// (plain_values; nothing else pays for it). Measured at 32 heads, 512 x 6,404, bf16: 158 us (202 with direct reads, 2,154 on the
-// FP32-FMA kernel that this form replaced).
+// nothing below 2^-36 of the row's maximum) bits of it: the probabilities of this path were fp32 before it used the tensor
+// core, and one 16-bit rounding would show. (The fp32 partials against 64 bits: bf16 1.6e-6 to 2.7e-6, fp16 5e-7 to 1.5e-6;
+// 2e-7 to 6e-7 on the FMA kernel that this form replaced.) Every tile takes the exact path, since scores that jump to -inf
+// are what a bias is for. A thread needs 128 consecutive values of its own row, which read directly would touch 32 lines a
+// load; each warp therefore copies 32 rows x 32 keys at a time into a swizzled buffer of its own, two pieces ahead of the
+// one it adds: a row's 128 bytes by eight lanes where rows are 16-byte aligned, one row at a time with 4 bytes a lane where
+// they are not (an odd number of keys). V keeps one stage then: its successor has the whole softmax to arrive in. An
+// infinity in V times the second half of P, which may be zero or negative, is NaN where the plain product is infinite: a row
+// that ends with NaN although its sum is finite is made again without halves (plain_values; nothing else pays for it).
+// Measured at 32 heads, bf16 (with direct reads; the FP32-FMA kernel that this form replaced):
+// 512 x 6,404 155 us (202; 2,120), 512 x 6,405 235 us (700; 2,104), 610 x 266 on 4 heads 20 us (42; 39).
 
 // 32 columns of one row's O over keys [key0, key1), as plain fp32 sums.
 template <bool IS_BF16>
@@ -109,12 +111,14 @@ __device__ __noinline__ void plain_values(float* o, const uint16_t* q, const uin
   }
 }
 
-template <bool IS_BF16, bool BIAS>
+// BIAS_COPY: bytes that a lane stages at a time; 0: no bias.
+template <bool IS_BF16, int BIAS_COPY>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
            const __grid_constant__ CUtensorMap tmV, const FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  constexpr bool BIAS = BIAS_COPY > 0;
   constexpr int NSV = BIAS ? 1 : FWD_NS;       // V stages
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (BIAS ? FWD_OFF_BAR_B : FWD_OFF_BAR));
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + FB_COUNT);
@@ -182,8 +186,21 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           brow = p.bias.base + blk * p.bias.s_blk + batch * p.bias.s_b +
                  ((kvs % p.hkv) * p.bias.g + prow / p.bias.sq) * p.bias.s_h + (prow % p.bias.sq) * p.bias.s_q;
       }
-      // Copies keys [col, col + 32) of the warp's 32 bias rows into piece `buf` (rows that do not exist as zeros).
+      // Copies keys [col, col + 32) of the warp's 32 bias rows into piece `buf` (rows that do not exist, and in the 4-byte form
+      // keys past the last valid one, as zeros).
       auto bias_copy = [&](int col, int buf) {
+        if constexpr (BIAS_COPY == 4) {
+#pragma unroll 8
+          for (int r = 0; r < 32; ++r) {
+            const float* src = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(brow), r));
+            const uint32_t dst = smem_u32(smem + FWD_OFF_BIAS + (warp * 2 + buf) * 4096 + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) +
+                                          (lane & 3) * 4);
+            const int bytes = src != nullptr && col + lane < valid ? 4 : 0;
+            src = bytes ? src + col + lane : p.bias.base;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+          }
+          return;
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int r = i * 4 + (lane >> 3), ch = lane & 7;
@@ -194,7 +211,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
         }
       };
-      auto bias_staged = [&](int j) { return p.bias_vec && j < n && (tile0 + j + 1) * 128 <= valid; };
+      auto bias_staged = [&](int j) {
+        return j < n && (BIAS_COPY == 16 ? (tile0 + j + 1) * 128 <= valid : p.bias_adjacent != 0);
+      };
       auto bias_commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
       if (BIAS && bias_staged(0)) {
         bias_copy(tile0 * 128, 0);
@@ -291,6 +310,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                   s[e][4 * i + 1] = __float_as_uint(fmaf(b.y, LOG2E, __uint_as_float(s[e][4 * i + 1]) * c));
                   s[e][4 * i + 2] = __float_as_uint(fmaf(b.z, LOG2E, __uint_as_float(s[e][4 * i + 2]) * c));
                   s[e][4 * i + 3] = __float_as_uint(fmaf(b.w, LOG2E, __uint_as_float(s[e][4 * i + 3]) * c));
+                }
+                if (BIAS_COPY == 4 && col0 + 128 > valid) {
+#pragma unroll
+                  for (int i = 0; i < 32; ++i)
+                    if (col0 + q * 32 + i >= valid) s[e][i] = 0xff800000u;
                 }
                 __syncwarp();
                 if (h == 0) bias_copy(col0 + (q + 2) * 32, e);
@@ -718,8 +742,9 @@ int launch_fwd_block(const lvx_shape& s, const FwdPlan& pl, const void* q, const
   p.q = q;
   p.k = k;
   p.v = v;
-  p.bias_vec = bias && bias->stride_kv == 1 && (reinterpret_cast<uintptr_t>(bias->bias) & 15) == 0 &&
-               ((bias->stride_block | bias->stride_b | bias->stride_h | bias->stride_q) & 3) == 0;
+  p.bias_adjacent = bias && bias->stride_kv == 1;
+  const bool aligned = (bias ? reinterpret_cast<uintptr_t>(bias->bias) & 15 : 1) == 0 &&
+                       ((bias->stride_block | bias->stride_b | bias->stride_h | bias->stride_q) & 3) == 0;
 
   dim3 grid(pl.m_blocks, qb * s.B * s.Hkv, pl.nsplit);
   cudaError_t e = cudaSuccess;
@@ -728,8 +753,17 @@ int launch_fwd_block(const lvx_shape& s, const FwdPlan& pl, const void* q, const
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) kern<<<grid, FWD_THREADS, smem, st>>>(tmQ, tmK, tmV, p);
   };
-  if (s.dtype == LVX_BF16) bias ? go(fwd_kernel<true, true>) : go(fwd_kernel<true, false>);
-  else bias ? go(fwd_kernel<false, true>) : go(fwd_kernel<false, false>);
+  // The 16-byte form wants aligned rows, and reads the ragged last tile directly; the 4-byte form stages that too, so it also
+  // takes shards of which the ragged tile is half or more (130 x 64: 18 us against 27), and keys that are not adjacent, which
+  // it reads directly. In one kernel the two cost the aligned case 4 %.
+  const bool wide_rows = aligned && p.bias_adjacent && s.Skv >= 256;
+  auto pick = [&](auto none, auto wide, auto narrow) {
+    if (!bias) go(none);
+    else if (wide_rows) go(wide);
+    else go(narrow);
+  };
+  if (s.dtype == LVX_BF16) pick(fwd_kernel<true, 0>, fwd_kernel<true, 16>, fwd_kernel<true, 4>);
+  else pick(fwd_kernel<false, 0>, fwd_kernel<false, 16>, fwd_kernel<false, 4>);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(fwd)");
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "fwd_kernel launch");

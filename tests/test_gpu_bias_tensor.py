@@ -170,3 +170,25 @@ def test_infinite_values_and_gradients(cuda_device, dtype):
             assert torch.equal(at(got), at(ref)), (name, at.__name__)
         fin = torch.isfinite(ref)
         assert ((got - ref)[fin].norm() / ref[fin].norm()).item() <= 1e-2, name
+
+
+@pytest.mark.parametrize("skv", [1, 31, 33, 64, 127, 128, 129, 252, 256, 257, 260, 383, 516])
+@pytest.mark.parametrize("valid", [None, 0.6])
+def test_staged_pieces_of_the_forward(cuda_device, skv, valid):
+    """Aligned and unaligned rows on both sides of 256 keys, with ends inside a piece of 32 keys. The bias is followed by NaN,
+    and its keys past the last valid one are NaN: neither may be seen."""
+    from lv_xattn_b200 import ops
+    B, H, Sq = 1, 2, 140
+    q, k, v, _ = orc.make_inputs(B, H, H, Sq, skv, 128, 80, torch.bfloat16)
+    n = None if valid is None else max(1, int(skv * valid))
+    buf = torch.full((H * Sq * skv + 4096,), float("nan"))
+    bias = buf[:H * Sq * skv].view(1, H, Sq, skv)
+    bias.copy_(torch.randn(1, H, Sq, skv, generator=torch.Generator().manual_seed(81)))
+    o_ref, lse_ref = orc.attention_fwd(q, k, v, SCALE, None if n is None else [n], bias=bias)
+    if n is not None:
+        bias[..., n:] = float("nan")
+    kvl = None if n is None else torch.tensor([n], dtype=torch.int32, device=cuda_device)
+    bias = buf.to(cuda_device)[:H * Sq * skv].view(1, H, Sq, skv)
+    o, lse = ops.fwd_block(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), SCALE, kv_valid_len=kvl, bias=bias)
+    _parity.assert_lse_close(lse.cpu().view(B, H, Sq), lse_ref, f"bias_pieces{skv}")
+    _parity.assert_close(o.float().cpu(), o_ref, "o", f"bias_pieces{skv}", *_parity.BF16["o"])
