@@ -78,7 +78,6 @@ fwd_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FR_OFF_BAR);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + FR_COUNT);
-  volatile int* poisoned = abort_flag + 1;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int split = blockIdx.x, slab = blockIdx.y;
@@ -98,11 +97,9 @@ fwd_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
       mbar_init(&bars[FR_EMPTY + s], FR_WARPS);
     }
     *abort_flag = 0;
-    *poisoned = word;
     fence_mbar_init();
   }
-  __syncthreads();
-  if (*poisoned != 0) return;
+  if (__syncthreads_or(word)) return;
 
   float* o_dst = p.o_part + (size_t(slab) * p.nsplit + split) * p.rows * 128;
   float* ml_dst = p.ml_part + (size_t(slab) * p.nsplit + split) * p.rows * 2;
